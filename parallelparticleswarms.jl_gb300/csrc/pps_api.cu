@@ -195,8 +195,9 @@ size_t swarm_device_bytes(const pps_problem* prob, int64_t n) { return swarm_lay
 // Points the swarm at device block `b` (layout L), copies the bounds, start
 // point and data asynchronously on s->stream and zeroes the rest.  Host
 // buffers are pageable, so each copy has left them when the call returns.
+// `extra` bytes behind the layout are zeroed too.
 static int swarm_setup(pps_swarm* s, const pps_problem* prob, int64_t n, uint64_t seed, uint32_t flags, char* b,
-                       const SwarmLayout& L) {
+                       const SwarmLayout& L, size_t extra = 0) {
   const int D = prob->dim;
   s->bytes = L.bytes;
   s->dv.X = reinterpret_cast<float*>(b + L.oX);
@@ -237,7 +238,7 @@ static int swarm_setup(pps_swarm* s, const pps_problem* prob, int64_t n, uint64_
     s->host_ub[d] = prob->ub ? prob->ub[d] : INFINITY;
     s->host_u0[d] = prob->u0 ? prob->u0[d] : 0.0f;
   }
-  PPS_CUDA(cudaMemsetAsync(b, 0, L.bytes, s->stream));
+  PPS_CUDA(cudaMemsetAsync(b, 0, L.bytes + extra, s->stream));
   PPS_CUDA(cudaMemcpyAsync(s->dv.lb, s->host_lb, sizeof(float) * D, cudaMemcpyHostToDevice, s->stream));
   PPS_CUDA(cudaMemcpyAsync(s->dv.ub, s->host_ub, sizeof(float) * D, cudaMemcpyHostToDevice, s->stream));
   PPS_CUDA(cudaMemcpyAsync(s->u0_dev, s->host_u0, sizeof(float) * D, cudaMemcpyHostToDevice, s->stream));
@@ -318,7 +319,8 @@ int swarm_create(const pps_problem* prob, int64_t n, uint64_t seed, uint32_t fla
   }
   const bool shard = nglobal > 0;
   const SwarmLayout L = swarm_layout(prob, n, shard);
-  cudaError_t e = cudaMalloc(&s->block, L.bytes);
+  const size_t xch = shard ? 0 : resident_exchange_bytes(prob->objective, prob->dim, n, prob->ncons, s->sm_count);
+  cudaError_t e = cudaMalloc(&s->block, L.bytes + xch);
   if (e != cudaSuccess) {
     delete s;
     return cuda_error(e, "cudaMalloc(swarm state)");
@@ -333,7 +335,8 @@ int swarm_create(const pps_problem* prob, int64_t n, uint64_t seed, uint32_t fla
       rc = cuda_error(e, "cudaEventCreate");
       break;
     }
-    if ((rc = swarm_setup(s, prob, n, seed, flags, static_cast<char*>(s->block), L))) break;
+    if ((rc = swarm_setup(s, prob, n, seed, flags, static_cast<char*>(s->block), L, xch))) break;
+    if (xch) s->xch_dev = reinterpret_cast<unsigned long long*>(static_cast<char*>(s->block) + L.bytes);
     if (shard) {
       s->shard = 1;
       s->dv.first = first;
@@ -521,10 +524,40 @@ static int run_steps(pps_swarm* s, int32_t maxiters, float c1, float c2, uint32_
   return PPS_OK;
 }
 
+// whether a run of this swarm keeps its state on chip (pps_resident.cu):
+// the swarm fits, its coefficients scale exactly (coef_scales), and the
+// TMA-staged step kernel has not been asked for
+static bool resident_applies(const pps_swarm* s, float c1, float c2, ResidentPlan* plan) {
+  if (s->shard || !s->owns_memory || !coef_scales(c1) || !coef_scales(c2)) return false;
+  if (sync_bulk_requested()) return false;
+  if (!resident_plan(s->objective, s->dv.dim, s->dv.n, s->dv.ncons, s->sm_count, plan)) return false;
+  return plan->blocks == 1 || s->xch_dev;
+}
+
 static int sync_like_run(pps_swarm* s, int32_t maxiters, float w, float wdamp, float c1, float c2,
                          float* device_ms, uint32_t run_flags) {
   int rc = check_run(s, maxiters, w, wdamp, c1, c2);
   if (rc) return rc;
+  ResidentPlan plan;
+  if (maxiters > 0 && resident_applies(s, c1, c2, &plan)) {
+    bool taken = false;
+    PPS_CUDA(cudaEventRecord(s->ev0, s->stream));
+    if ((rc = launch_resident(s, plan, maxiters, w, wdamp, c1, c2,
+                              (run_flags & PPS_FLAG_GBEST_FROM_POSITION) ? 1 : 0, &taken)))
+      return rc;
+    if (taken) {
+      PPS_CUDA(cudaEventRecord(s->ev1, s->stream));
+      unsigned int status = 0;
+      if (plan.blocks > 1)
+        PPS_CUDA(cudaMemcpyAsync(&status, &s->dv.st->status, sizeof(status), cudaMemcpyDeviceToHost, s->stream));
+      PPS_CUDA(cudaStreamSynchronize(s->stream));
+      if ((rc = finish_timing(s, device_ms))) return rc;
+      s->t += (uint32_t)maxiters;
+      if (status & kStatusResidentTimeout)
+        return set_error(PPS_ETIMEOUT, "the resident run timed out waiting for another block's best");
+      return PPS_OK;
+    }
+  }
   if ((rc = launch_set_iter(s, s->t, w, wdamp))) return rc;
   PPS_CUDA(cudaEventRecord(s->ev0, s->stream));
   if ((rc = run_steps(s, maxiters, c1, c2, run_flags))) return rc;

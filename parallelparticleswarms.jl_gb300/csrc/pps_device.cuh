@@ -119,6 +119,50 @@ __device__ __forceinline__ Rand4 philox4x32_10(uint32_t c0, uint32_t c1, uint32_
   return Rand4{c0, c1, c2, c3};
 }
 
+// The update draws of one particle with everything that does not depend on
+// the dim pair computed ahead: in the first three rounds of counter
+// {particle, j, t, tag} five of the six products depend on the particle or
+// on the particle and the iteration alone, so a loop over pairs (and over
+// iterations) carries them instead of redoing them: 16 wide multiplications a
+// call for 20.  The words are those of philox4x32_10(particle, j, t, kTagStep, K).
+struct PhiloxParticle {
+  uint32_t a1, b1, l0;
+  __device__ __forceinline__ void start(uint32_t particle, const PhiloxKeys& K) {
+    const uint64_t p0 = (uint64_t)0xD2511F53u * (uint64_t)particle;
+    const uint64_t q1 = (uint64_t)0xCD9E8D57u * (uint64_t)((uint32_t)(p0 >> 32) ^ kTagStep ^ K.k[1]);
+    a1 = (uint32_t)(q1 >> 32) ^ K.k[2];
+    b1 = (uint32_t)q1 ^ K.k[4];
+    l0 = (uint32_t)p0 ^ K.k[3];
+  }
+};
+struct PhiloxIteration {
+  uint32_t h1, sh, sl, l0, b1;
+  __device__ __forceinline__ void start(const PhiloxParticle& P, uint32_t t, const PhiloxKeys& K) {
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * (uint64_t)t;
+    const uint64_t s0 = (uint64_t)0xD2511F53u * (uint64_t)(P.a1 ^ (uint32_t)p1);
+    h1 = (uint32_t)(p1 >> 32) ^ K.k[0];
+    sh = (uint32_t)(s0 >> 32) ^ K.k[5];
+    sl = (uint32_t)s0;
+    l0 = P.l0;
+    b1 = P.b1;
+  }
+  __device__ __forceinline__ Rand4 draw(uint32_t j, const PhiloxKeys& K) const {
+    const uint64_t q0 = (uint64_t)0xD2511F53u * (uint64_t)(h1 ^ j);
+    const uint64_t s1 = (uint64_t)0xCD9E8D57u * (uint64_t)((uint32_t)(q0 >> 32) ^ l0);
+    uint32_t c0 = (uint32_t)(s1 >> 32) ^ b1, c1 = (uint32_t)s1, c2 = sh ^ (uint32_t)q0, c3 = sl;
+#pragma unroll
+    for (int r = 3; r < 10; ++r) {
+      const uint64_t p0 = (uint64_t)0xD2511F53u * (uint64_t)c0;
+      const uint64_t p1 = (uint64_t)0xCD9E8D57u * (uint64_t)c2;
+      c0 = (uint32_t)(p1 >> 32) ^ c1 ^ K.k[2 * r];
+      c1 = (uint32_t)p1;
+      c2 = (uint32_t)(p0 >> 32) ^ c3 ^ K.k[2 * r + 1];
+      c3 = (uint32_t)p0;
+    }
+    return Rand4{c0, c1, c2, c3};
+  }
+};
+
 __device__ __forceinline__ float u01(uint32_t bits) {
   return __fmul_rn(__uint2float_rn(bits >> 8), 0x1p-24f);
 }
@@ -367,6 +411,21 @@ __device__ __forceinline__ float velocity(float x, float v, float p, float g, fl
   const float c = __fmul_rn(__fmul_rn(c2, r2), __fsub_rn(g, x));
   return __fadd_rn(__fadd_rn(a, b), c);
 }
+
+// The same update from the draws' 24-bit integers m = bits >> 8, with c1s =
+// c1 2^-24 and c2s = c2 2^-24: c1 (m 2^-24) and (c1 2^-24) m are the same
+// real product, so they round to the same value wherever c1s is exact (see
+// coef_scales), and the draw's own multiplication by 2^-24 goes.
+__device__ __forceinline__ float draw24(uint32_t bits) { return __uint2float_rn(bits >> 8); }
+__device__ __forceinline__ float velocity24(float x, float v, float p, float g, float w, float c1s, float c2s,
+                                            uint32_t r1, uint32_t r2) {
+  const float a = __fmul_rn(w, v);
+  const float b = __fmul_rn(__fmul_rn(c1s, draw24(r1)), __fsub_rn(p, x));
+  const float c = __fmul_rn(__fmul_rn(c2s, draw24(r2)), __fsub_rn(g, x));
+  return __fadd_rn(__fadd_rn(a, b), c);
+}
+// whether c 2^-24 is exact (c is 0 or large enough that it stays normal)
+__host__ __device__ inline bool coef_scales(float c) { return c == 0.0f || c >= 0x1p-100f || c <= -0x1p-100f; }
 
 // ---------------------------------------------------------------- objectives
 // Objective parameters, passed by value to every kernel.

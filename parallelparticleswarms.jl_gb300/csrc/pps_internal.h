@@ -59,6 +59,8 @@ struct pps_swarm {
   const unsigned char* shard_records = nullptr;  // shard: every shard's record after the exchange
   int shard_nrecords = 0;
   int bounded_waits = 0;      // 1: a kernel with bounded mbarrier waits ran (a timeout sets IterState::status)
+  unsigned long long* xch_dev = nullptr;  // exchange words of the resident run's grid form (behind the state in block)
+  uint32_t xch_seq = 0;       // exchanges made so far: the sequence number of the last one
 };
 
 namespace pps {
@@ -90,6 +92,18 @@ int sync_bulk_prepare(pps_swarm* s, int* blocks_per_sm);
 // IterState::status after the swarm's stream is idle), else PPS_OK
 int check_device_status(pps_swarm* s);
 int launch_sync_step_bulk(pps_swarm* s, float c1, float c2, bool* taken);
+bool sync_bulk_requested();  // PPS_SYNC_KERNEL=bulk
+// a whole run in one launch with the state in shared memory (pps_resident.cu)
+struct ResidentPlan {
+  int blocks, threads, chunk, groups;
+  bool split;
+  size_t smem;
+};
+bool resident_plan(int objective, int dim, int64_t n, int ncons, int sm_count, ResidentPlan* p);
+size_t resident_exchange_bytes(int objective, int dim, int64_t n, int ncons, int sm_count);
+// *taken false: the device could not hold the grid, nothing was launched
+int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w, float wdamp, float c1, float c2,
+                    int from_position, bool* taken);
 int local_field(pps_swarm* s, int32_t field, float** dev, int* rows);
 // ODE-fit objectives (pps_ode.cu)
 int ode_check(const pps_problem* prob);

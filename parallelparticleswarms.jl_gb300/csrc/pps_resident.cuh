@@ -1,0 +1,378 @@
+// pps_resident.cuh -- a whole synchronous run of one swarm inside one launch,
+// the swarm's state resident in shared memory.
+//
+// Same particles, draws, operation order, strict `<`, lowest-index argmin and
+// global best as one k_sync_step launch per iteration (src/kernels.jl:127-177,
+// src/lowerlevel_solve.jl:1-65), so the state after a run is bit-identical.
+//
+// What bounds the launch-per-iteration form for a swarm that fits the chip is
+// neither bandwidth nor arithmetic but latency: a launch per iteration (about
+// 5 us), a thread walking every dim of its particles in sequence with an L2
+// round trip per pair, and few warps.  Here:
+//   - each block owns `chunk` consecutive particles for the whole run; x, v
+//     and pbest live in its shared memory as float2 (dims 2j, 2j+1) at
+//     [j][particle], so a pair is one 64-bit access per array;
+//   - with fewer particles than threads, `groups` threads share a particle's
+//     pairs (SPLIT): they move the coordinates and leave the costly objective
+//     terms (the cosines) in shared memory, and one thread per particle then
+//     sums the terms in dim order -- the order the streaming accumulators use;
+//   - blocks agree on the global best once per iteration through 64-bit words
+//     in global memory that carry a 32-bit value and the 32-bit sequence
+//     number of the exchange, so a reader that sees the number has the value
+//     and no fence or counter stands between them.  Every block posts its own
+//     best and that particle's vector together; one warp per block gathers the
+//     posts.  Two buffers alternate: a block can only be one exchange ahead of
+//     another, since it needs the other's post to go on.  The grid is a
+//     cooperative launch, so every block is resident.
+// The wait for a post is bounded (poll_limit polls); a wait that gives up sets
+// IterState::status bit 3 and the block leaves the loop.
+#pragma once
+#include "pps_publish.cuh"
+
+namespace pps {
+
+struct ResidentArgs {
+  int chunk;          // particles of a block
+  int groups;         // threads that share a particle's pairs
+  int iters;
+  uint32_t t0;
+  float w0, wdamp;
+  float c1s, c2s;     // c1 2^-24, c2 2^-24 (velocity24)
+  int from_position;
+  uint32_t seq0;      // sequence number before the first exchange
+  unsigned int poll_limit;
+  unsigned long long* xch;  // exchange of a grid of several blocks: two buffers of resident_words
+};
+
+// objectives whose terms are computed while moving in the SPLIT form
+template <int OBJ>
+constexpr bool kTermsMoved = OBJ == kRastrigin || OBJ == kAckley;
+
+constexpr int kResidentMaxThreads = 1024;
+
+// shared memory of a block: bounds (float4 per pair), g (float2 per pair),
+// x, v, pbest (float2 per pair and particle), the moved terms, pcost, flags
+__host__ __device__ inline size_t resident_smem(int dim, int chunk, bool terms) {
+  const size_t np = (size_t)(dim + 1) / 2;
+  return 16 * np + 8 * np + 8 * np * (size_t)chunk * (terms ? 4 : 3) + 4 * (size_t)chunk +
+         ((size_t)chunk + 15) / 16 * 16;
+}
+
+// 64-bit words of an exchange's one buffer: each block's key (two words:
+// cost and index), packed so a warp polls whole lines, then the vectors; even,
+// so the second buffer's keys too start on the 16 bytes their loads need
+__host__ __device__ inline size_t resident_words(int blocks, int dim) {
+  return ((size_t)blocks * (2 + (size_t)dim) + 1) / 2 * 2;
+}
+
+__device__ __forceinline__ unsigned long long resident_word(uint32_t value, uint32_t seq) {
+  return ((unsigned long long)value << 32) | (unsigned long long)seq;
+}
+
+// minimum of the warp's 64-bit keys by two 32-bit hardware reductions
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+  const uint32_t hi = (uint32_t)(k >> 32), lo = (uint32_t)k;
+  const uint32_t m = __reduce_min_sync(0xffffffffu, hi);
+  const uint32_t i = __reduce_min_sync(0xffffffffu, hi == m ? lo : 0xffffffffu);
+  return ((unsigned long long)m << 32) | (unsigned long long)i;
+}
+
+// one coordinate's term of an objective that is a sum of them (kTermsMoved)
+template <int OBJ>
+__device__ __forceinline__ float moved_term(const ObjParams& op, float x) {
+  if constexpr (OBJ == kRastrigin) return __fsub_rn(__fmul_rn(x, x), __fmul_rn(prm(op, 0, 10.0f), cos2pi(x)));
+  if constexpr (OBJ == kAckley) return cos2pi(__fmul_rn(prm(op, 2, 1.0f), x));
+  return 0.0f;
+}
+
+__device__ __forceinline__ void post_word(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// waits for the word of exchange `seq`; false after `limit` polls without it
+__device__ __forceinline__ bool await_word(const unsigned long long* p, uint32_t seq, unsigned int limit,
+                                           uint32_t* value) {
+  for (unsigned int n = 0; n < limit; ++n) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    if ((uint32_t)v == seq) {
+      *value = (uint32_t)(v >> 32);
+      return true;
+    }
+  }
+  return false;
+}
+// The lowest of the blocks' keys of exchange `seq`, by one warp: each lane
+// polls its up to kPollSlots keys with all loads in flight, so a round costs
+// one L2 round trip whatever the number of blocks (one word after the other:
+// 4.8 us an iteration at 152 blocks for 2.0).  ok: every key arrived.
+constexpr int kPollSlots = 5;  // 160 blocks a round
+__device__ __forceinline__ unsigned long long await_keys(const unsigned long long* keys, int blocks, uint32_t seq,
+                                                         unsigned int limit, bool* ok) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long best = ~0ull;
+  for (int base = 0; base < blocks; base += 32 * kPollSlots) {
+    unsigned int missing = 0u;
+#pragma unroll
+    for (int i = 0; i < kPollSlots; ++i)
+      if (base + 32 * i + lane < blocks) missing |= 1u << i;
+    for (unsigned int n = 0; missing && n < limit; ++n) {
+      unsigned long long a[kPollSlots], b[kPollSlots];
+#pragma unroll
+      for (int i = 0; i < kPollSlots; ++i) {
+        a[i] = b[i] = 0ull;
+        if (missing & (1u << i)) {
+          const unsigned long long* p = keys + 2 * (size_t)(base + 32 * i + lane);
+          asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(a[i]), "=l"(b[i]) : "l"(p) : "memory");
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kPollSlots; ++i) {
+        if ((missing & (1u << i)) && (uint32_t)a[i] == seq && (uint32_t)b[i] == seq) {
+          missing &= ~(1u << i);
+          const unsigned long long k = (a[i] & 0xffffffff00000000ull) | (b[i] >> 32);
+          best = k < best ? k : best;
+        }
+      }
+    }
+    if (missing) *ok = false;
+  }
+  return warp_min_key(best);
+}
+
+template <int OBJ, bool SPLIT, bool CONS>
+__device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams& op, const PhiloxKeys& keys,
+                                             const ResidentArgs& a) {
+  static_assert(SPLIT || !CONS, "the constrained form sums in its own phase");
+  extern __shared__ __align__(16) float rsm[];
+  __shared__ unsigned long long red[2][32];
+  __shared__ unsigned long long win_s;
+  __shared__ int bail;
+  const int D = s.dim, np = (D + 1) >> 1, chunk = a.chunk;
+  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
+  const int64_t first = (int64_t)blockIdx.x * chunk;
+  int cnt = (int)(s.n - first < (int64_t)chunk ? s.n - first : (int64_t)chunk);
+  cnt = cnt < 0 ? 0 : cnt;
+  constexpr bool TERMS = SPLIT && kTermsMoved<OBJ>;
+
+  float4* bnd = reinterpret_cast<float4*>(rsm);
+  float2* g2 = reinterpret_cast<float2*>(bnd + np);
+  float2* X = g2 + np;
+  float2* V = X + np * chunk;
+  float2* P = V + np * chunk;
+  float2* TM = P + np * chunk;
+  float* pcost = reinterpret_cast<float*>(TM + (TERMS ? np * chunk : 0));
+  unsigned char* flag = reinterpret_cast<unsigned char*>(pcost + chunk);
+  float* gs = reinterpret_cast<float*>(g2);
+
+  for (int j = tid; j < np; j += T) {
+    const bool two = 2 * j + 1 < D;
+    g2[j] = make_float2(s.g[2 * j], two ? s.g[2 * j + 1] : 0.0f);
+    bnd[j] = make_float4(s.lb[2 * j], s.ub[2 * j], two ? s.lb[2 * j + 1] : 0.0f, two ? s.ub[2 * j + 1] : 0.0f);
+  }
+  for (int p = tid; p < cnt; p += T) {
+    pcost[p] = s.pcost[first + p];
+    flag[p] = s.flag[first + p];
+  }
+  if (tid == 0) bail = 0;
+  for (int p = lane; p < cnt; p += 32) {  // a warp per pair row
+    for (int j = warp; j < np; j += nw) {
+      const int64_t o = (int64_t)(2 * j) * s.npad + first + p;
+      const bool two = 2 * j + 1 < D;
+      X[j * chunk + p] = make_float2(s.X[o], two ? s.X[o + s.npad] : 0.0f);
+      V[j * chunk + p] = make_float2(s.V[o], two ? s.V[o + s.npad] : 0.0f);
+      P[j * chunk + p] = make_float2(s.P[o], two ? s.P[o + s.npad] : 0.0f);
+    }
+  }
+  __syncthreads();
+
+  const int G = SPLIT ? a.groups : 1;
+  int p0 = tid, g0 = 0;
+  if (SPLIT && G > 1) {
+    g0 = tid / chunk;
+    p0 = g0 < G ? tid - g0 * chunk : cnt;
+  }
+  const int stride = (SPLIT && G > 1) ? chunk : T;  // one particle per thread when pairs are shared
+  float w = a.w0;
+  unsigned long long win = ~0ull, prev = ~0ull;
+  bool have_prev = false;
+  PhiloxParticle pp;
+  pp.start((uint32_t)(first + p0), keys);
+
+  for (int it = 0; it < a.iters; ++it) {
+    const uint32_t t = a.t0 + (uint32_t)it;
+    const int par = it & 1;
+    unsigned long long best = ~0ull;
+    auto settle = [&](int p, float c) {
+      const float pc = pcost[p];
+      const bool imp = c < pc;  // strict <, src/kernels.jl:21-24
+      const float npc = imp ? c : pc;
+      if (imp) pcost[p] = c;
+      flag[p] = imp ? 1 : 0;
+      if (it == a.iters - 1) s.cost[first + p] = c;
+      const unsigned long long k = argmin_key(npc, (uint32_t)(first + p));
+      best = k < best ? k : best;
+    };
+    // ---- move (src/kernels.jl:1-26)
+    for (int p = p0; p < cnt; p += stride) {
+      if (chunk > T) pp.start((uint32_t)(first + p), keys);  // else the thread's one particle
+      PhiloxIteration pi;
+      pi.start(pp, t, keys);
+      const bool fl = flag[p] != 0;
+      Acc<OBJ> acc;
+#pragma unroll 1
+      for (int j = g0; j < np; j += G) {
+        const Rand4 r = pi.draw((uint32_t)j, keys);
+        const int o = j * chunk + p;
+        float2 x = X[o], v = V[o], q = P[o];
+        if (fl) {  // the personal-best copy deferred from the last iteration
+          q = x;
+          P[o] = q;
+        }
+        const float2 gd = g2[j];
+        const float4 b = bnd[j];
+        v.x = velocity24(x.x, v.x, q.x, gd.x, w, a.c1s, a.c2s, r.a, r.b);
+        v.y = velocity24(x.y, v.y, q.y, gd.y, w, a.c1s, a.c2s, r.c, r.d);
+        x.x = clamp_lb_ub(__fadd_rn(x.x, v.x), b.x, b.y);
+        x.y = clamp_lb_ub(__fadd_rn(x.y, v.y), b.z, b.w);
+        X[o] = x;
+        V[o] = v;
+        if constexpr (!SPLIT) {
+          acc.add(op, 2 * j, x.x);
+          if (2 * j + 1 < D) acc.add(op, 2 * j + 1, x.y);
+        } else if constexpr (TERMS) {
+          TM[o] = make_float2(moved_term<OBJ>(op, x.x), moved_term<OBJ>(op, x.y));
+        }
+      }
+      if constexpr (!SPLIT) settle(p, finalize<OBJ>(op, acc.s1, acc.s2));
+    }
+    // ---- sum the terms in dim order
+    if constexpr (SPLIT) {
+      __syncthreads();
+      for (int p = tid; p < cnt; p += T) {
+        Acc<OBJ> acc;
+        ConsAcc ca;
+        if constexpr (CONS) ca.start(s.cons, s.ncons, D);
+        auto add = [&](int d, float x, float term) {
+          if constexpr (OBJ == kRastrigin) {
+            acc.s1 = __fadd_rn(acc.s1, term);
+          } else if constexpr (OBJ == kAckley) {
+            acc.s1 = __fadd_rn(acc.s1, __fmul_rn(x, x));
+            acc.s2 = __fadd_rn(acc.s2, term);
+          } else {
+            acc.add(op, d, x);
+          }
+          if constexpr (CONS) ca.add(s.cons, s.ncons, D, d, x);
+        };
+        const int full = D >> 1;
+#pragma unroll 4
+        for (int j = 0; j < full; ++j) {
+          const float2 x = X[j * chunk + p], m = TERMS ? TM[j * chunk + p] : x;
+          add(2 * j, x.x, m.x);
+          add(2 * j + 1, x.y, m.y);
+        }
+        if (D & 1) {
+          const float2 x = X[full * chunk + p], m = TERMS ? TM[full * chunk + p] : x;
+          add(D - 1, x.x, m.x);
+        }
+        float c = finalize<OBJ>(op, acc.s1, acc.s2);
+        if constexpr (CONS) c = __fadd_rn(c, penalty(ca, s.ncons, __uint2float_rn((uint32_t)(first + p) + 2u)));
+        settle(p, c);
+      }
+    }
+    // ---- the block's best
+    best = warp_min_key(best);
+    if (lane == 0) red[par][warp] = best;
+    __syncthreads();
+    const unsigned long long mine = warp_min_key(lane < nw ? red[par][lane] : ~0ull);
+    const int lp = (int)((int64_t)(uint32_t)mine - first);  // its particle (meaningless when mine is ~0)
+    const bool none = mine == ~0ull;
+    const float* src = nullptr;  // its vector: the position if it improved just now, else the personal best
+    if (!none) src = reinterpret_cast<const float*>((a.from_position || flag[lp]) ? X : P);
+    // ---- agree on the global best
+    const uint32_t seq = a.seq0 + 1u + (uint32_t)it;
+    const int nb = (int)gridDim.x;
+    unsigned long long* kw = a.xch + (size_t)par * resident_words(nb, D);  // keys
+    unsigned long long* vw = kw + 2 * (size_t)nb;                          // vectors
+    if (nb == 1) {
+      win = mine;
+      for (int d = tid; d < D; d += T) gs[d] = src[2 * ((d >> 1) * chunk + lp) + (d & 1)];
+    } else {
+      if (tid == 0) {
+        post_word(kw + 2 * (size_t)blockIdx.x, resident_word((uint32_t)(mine >> 32), seq));
+        post_word(kw + 2 * (size_t)blockIdx.x + 1, resident_word((uint32_t)mine, seq));
+      }
+      if (!none)
+        for (int d = tid; d < D; d += T)
+          post_word(vw + (size_t)blockIdx.x * D + d,
+                    resident_word(__float_as_uint(src[2 * ((d >> 1) * chunk + lp) + (d & 1)]), seq));
+    }
+    if (nb > 1 && warp == 0) {
+      bool ok = true;
+      const unsigned long long k = await_keys(kw, nb, seq, a.poll_limit, &ok);
+      ok = __all_sync(0xffffffffu, ok);
+      // nobody's personal best beat the last global best: its vector stands
+      if (ok && (a.from_position || !have_prev || k != prev)) {
+        const unsigned long long* v = vw + (size_t)((int64_t)(uint32_t)k / chunk) * D;
+        for (int d = lane; d < D && ok; d += 32) {
+          uint32_t bits = 0u;
+          ok = await_word(v + d, seq, a.poll_limit, &bits);
+          gs[d] = __uint_as_float(bits);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+      }
+      if (lane == 0) {
+        win_s = k;
+        if (!ok) {
+          bail = 1;
+          atomicOr(&s.st->status, kStatusResidentTimeout);
+        }
+      }
+    }
+    __syncthreads();
+    if (nb > 1) {
+      win = win_s;
+      if (bail) return;
+      prev = win;
+      have_prev = true;
+    }
+    w = __fmul_rn(w, a.wdamp);
+  }
+
+  // ---- the state back to global memory, personal bests canonical
+  for (int p = lane; p < cnt; p += 32) {
+    const bool fl = flag[p] != 0;
+    for (int j = warp; j < np; j += nw) {
+      const int64_t o = (int64_t)(2 * j) * s.npad + first + p;
+      const float2 x = X[j * chunk + p], v = V[j * chunk + p];
+      const float2 q = fl ? x : P[j * chunk + p];
+      s.X[o] = x.x;
+      s.V[o] = v.x;
+      s.P[o] = q.x;
+      if (2 * j + 1 < D) {
+        s.X[o + s.npad] = x.y;
+        s.V[o + s.npad] = v.y;
+        s.P[o + s.npad] = q.y;
+      }
+    }
+  }
+  for (int p = tid; p < cnt; p += T) {
+    s.pcost[first + p] = pcost[p];
+    s.flag[first + p] = 0;
+  }
+  if (blockIdx.x == 0) {
+    for (int d = tid; d < D; d += T) s.g[d] = gs[d];
+    if (tid == 0) {
+      const uint32_t o = (uint32_t)(win >> 32);
+      s.st->gcost = __uint_as_float((o & 0x80000000u) ? (o ^ 0x80000000u) : ~o);
+      s.st->gidx = (uint32_t)win;
+      s.st->key = ~0ull;
+      s.st->count = 0u;
+      s.st->tile_next = 0u;
+      s.st->t = a.t0 + (uint32_t)a.iters;
+      s.st->w = w;
+      s.st->wdamp = a.wdamp;
+    }
+  }
+}
+
+}  // namespace pps

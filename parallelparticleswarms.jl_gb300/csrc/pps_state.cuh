@@ -23,6 +23,9 @@ struct IterState {
   unsigned int pad[6];
 };
 
+// IterState::status bit of a resident run whose wait for another block's post gave up
+constexpr unsigned int kStatusResidentTimeout = 8u;
+
 // Swarm state in HBM (structure of arrays, particle index fastest):
 //   X, V, P   [dim][npad] float   position, velocity, personal best
 //   pcost     [npad] float        personal best cost

@@ -299,6 +299,8 @@ static bool bulk_enabled() {
   return on;
 }
 
+bool sync_bulk_requested() { return bulk_enabled(); }
+
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 using BulkKernel = void (*)(SwarmDev, ObjParams, PhiloxKeys, float, float, int, int);
