@@ -620,9 +620,9 @@ size_t batch_smem_bytes(int maxdim, int data_floats, int64_t maxchunk) {
 }
 
 // Shape limits: PPS_BATCH_MAX_CLUSTER (1..16, default 4) caps the CTAs a swarm
-// is split over, PPS_ODE_THREADS (256/512/1024, default 512) is the largest
-// block of an ODE-fit CTA.  They change how work is placed, never what is
-// computed.  Clusters above 8 CTAs are a non-portable size.
+// is split over (ODE fits: kOdeMaxCluster), PPS_ODE_THREADS (128..1024, default
+// 128) is the block of an ODE-fit CTA.  They change how work is placed, never
+// what is computed.  Clusters above 8 CTAs are a non-portable size.
 static int env_int(const char* name, int dflt, int lo, int hi) {
   const char* e = getenv(name);
   const int v = e ? atoi(e) : dflt;
@@ -644,24 +644,23 @@ static int batch_dim_ref() {
   return v;
 }
 static int ode_threads() {
-  static const int v = env_int("PPS_ODE_THREADS", 512, 256, 1024);
+  static const int v = env_int("PPS_ODE_THREADS", 128, 128, 1024) / 32 * 32;
   return v;
 }
+constexpr int kOdeMaxCluster = 8;
 
 LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread) {
   LaunchGroup g{};
   const int cmax = max_cluster();
   if (is_ode(d.objective)) {
     g.kind = 1;
-    // two particles per thread and trip (the packed RK4 losses): the
-    // smallest power-of-two block from 128 that covers half the particles
-    const int tmax = ode_threads();
-    const int64_t half = (d.n + 1) / 2;
-    int T = 128;
-    while (T < half && T < 1024 && 2 * T <= tmax) T *= 2;
-    g.T = T;
+    // two particles per thread and trip (the packed RK4 losses); CTAs of one
+    // warp per scheduler spread a fit over more SMs than few large ones do
+    // (PPS_ODE_THREADS): 128 mixed fits, 512 threads and clusters of 4: 98 ms,
+    // 128 threads and clusters of 8: 58 ms
+    g.T = ode_threads();
     const int64_t c = (d.n + 2 * (int64_t)g.T - 1) / (2 * (int64_t)g.T);
-    g.C = (int)(c < cmax ? c : cmax);
+    g.C = (int)(c < kOdeMaxCluster ? c : kOdeMaxCluster);
   } else {
     g.kind = 0;
     g.T = threads;
@@ -789,6 +788,7 @@ struct pps_batch {
   BatchSwarm* ddescs = nullptr;
   int* dorder = nullptr;
   size_t dcap = 0;
+  OdeTeams* teams = nullptr;  // ODE fits alone: their units' tables
   int tuned_threads = 0, tuned_ppt = 0, tuned_spread = 8;
   int last_threads = 0, last_ppt = 0, last_spread = 8;
   int last_groups = 0, last_max_cluster = 0;
@@ -951,6 +951,7 @@ int pps_batch_destroy(pps_batch* b) {
   if (b->arena) cudaFree(b->arena);
   if (b->ddescs) cudaFree(b->ddescs);
   if (b->dorder) cudaFree(b->dorder);
+  ode_teams_destroy(b->teams);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -983,6 +984,26 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
   int rc = prepare(b);
   if (rc) return rc;
   const int ns = (int)b->descs.size();
+  bool all_ode = true;
+  for (const auto& d : b->descs) all_ode = all_ode && is_ode(d.objective);
+  if (all_ode) {  // ODE fits alone have a form of their own, with nothing to tune
+    if (!b->teams && !(b->teams = ode_teams_create())) return set_error(PPS_ENOMEM, "host allocation failed");
+    bool taken = false;
+    unsigned int *word = nullptr, timed_out = 0;
+    PPS_CUDA(cudaEventRecord(b->ev0, b->stream));
+    if ((rc = ode_teams_launch(b->teams, b->stream, b->descs, b->ddescs, b->sm_count, &taken, &word))) return rc;
+    if (taken) {
+      PPS_CUDA(cudaEventRecord(b->ev1, b->stream));
+      PPS_CUDA(cudaMemcpyAsync(&timed_out, word, sizeof(timed_out), cudaMemcpyDeviceToHost, b->stream));
+      PPS_CUDA(cudaStreamSynchronize(b->stream));
+      if (device_ms) PPS_CUDA(cudaEventElapsedTime(device_ms, b->ev0, b->ev1));
+      if (timed_out) return set_error(PPS_ETIMEOUT, "the batch timed out waiting for a fit's iteration");
+      b->last_threads = 128;
+      b->last_ppt = 1;
+      b->ran = true;
+      return PPS_OK;
+    }
+  }
   // autotune the block shape for this batch shape (cached), unless PPS_BATCH_SHAPE
   // pins it for every batch ("threads,ppt,spread", e.g. "256,2,2": reproducible
   // profiles, since the autotuner's timings are not representative under a profiler)
@@ -998,11 +1019,7 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
     if (!threads) {
       // time each candidate on this batch with a few iterations per swarm
       std::vector<BatchSwarm> saved = b->descs;
-      bool all_ode = true;
-      for (auto& d : b->descs) {
-        d.maxiters = std::min(d.maxiters, 4);
-        all_ode = all_ode && is_ode(d.objective);
-      }
+      for (auto& d : b->descs) d.maxiters = std::min(d.maxiters, 4);
       PPS_CUDA(cudaMemcpyAsync(b->ddescs, b->descs.data(), sizeof(BatchSwarm) * ns, cudaMemcpyHostToDevice, b->stream));
       // block size x particles per thread x particles per thread per
       // iteration: a batch of few swarms runs faster spread over more CTAs

@@ -61,6 +61,15 @@ LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread
 // group, longest estimated work first inside each group
 void batch_plan(const std::vector<BatchSwarm>& descs, int threads, int ppt, std::vector<int>* order,
                 std::vector<LaunchGroup>* groups, int spread = 8);
+// a batch of ODE fits alone, its units of work placed on the SMs by cost
+// (pps_ode_teams.cu): every fit's whole run in one cooperative launch.  *taken
+// false: nothing was launched (the device cannot hold the grid); else
+// *error_word is a device word, nonzero after the run if a wait gave up.
+struct OdeTeams;
+OdeTeams* ode_teams_create();
+void ode_teams_destroy(OdeTeams* t);
+int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSwarm>& descs, const BatchSwarm* ddescs,
+                     int sm_count, bool* taken, unsigned int** error_word);
 // launch one group: descs[dorder[g.offset + k]], k < g.count, on `stream`
 int batch_launch_group(cudaStream_t stream, const BatchSwarm* ddescs, const int* dorder, const LaunchGroup& g,
                        int ppt);

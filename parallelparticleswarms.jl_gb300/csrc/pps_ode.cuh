@@ -171,7 +171,7 @@ __device__ __forceinline__ float2 ode_loss2(const float* pa, const float* pb, co
   float2 e0 = add(dup(data[0]), neg(u0), one), e1 = add(dup(data[1]), neg(u1), one);
   float2 acc = add(mul(e0, e0), mul(e1, e1), one);
   for (int m = 1; m < c.nsaves; ++m) {
-#pragma unroll 2
+#pragma unroll 5  // the packed loop's trips: 1 / 2 / 5 steps 59.2 / 54.6 / 52.2 ms for 128 batched fits
     for (int k = 0; k < c.save_every; ++k) {
       float2 k1a, k1b, k2a, k2b, k3a, k3b, k4a, k4b;
       rhs<MODEL>(p, l, one, u0, u1, k1a, k1b);
