@@ -269,6 +269,26 @@ __device__ __forceinline__ float cos2pi(float x) {
   const float c = __fmaf_rn(p, __fmul_rn(z, q), __fmul_rn(4.0f, p));
   return __uint_as_float(__float_as_uint(c) ^ (odd << 31));
 }
+// cos2pi for |x| < 2^126, the same value bit for bit in 14 instructions and one
+// conversion for 18 and two: x = m + f with m = rint(x) and f exact, h =
+// min(|f|, 1/2 - |f|) = a / 2 (exact: 1/2 - |f| is only taken where |f| >=
+// 1/4), and cos(2 pi x) is negative exactly where |f| > 1/4 (n odd above).
+// The polynomial is cos2pi's with z = 4 h^2 and its powers of two moved into
+// the constants and the last step, which changes no rounding: 4p = 1 - 16 h^2
+// is one fused multiply-add, c = 4p (z q / 4) + 4p.  Beyond 2^126 cos2pi's 2x
+// overflows and it returns NaN; this form would not.
+constexpr float kCosBoxLimit = 0x1p+126f;
+__device__ __forceinline__ float cos2pi_box(float x) {
+  const float f = fabsf(__fsub_rn(x, rintf(x)));
+  const float h = fminf(f, __fsub_rn(0.5f, f));
+  const float z = __fmul_rn(h, h);
+  float q = __fmaf_rn(64.0f * kCosP3, z, 16.0f * kCosP2);
+  q = __fmaf_rn(q, z, 4.0f * kCosP1);
+  q = __fmaf_rn(q, z, kCosP0);
+  const float p4 = __fmaf_rn(__fmul_rn(-16.0f, h), h, 1.0f);
+  const float c = __fmaf_rn(p4, __fmul_rn(z, q), p4);
+  return __uint_as_float((__float_as_uint(c) & 0x7fffffffu) | (__float_as_uint(__fsub_rn(0.25f, f)) & 0x80000000u));
+}
 __device__ __forceinline__ float sin2pi(float x) {
   const float y = __fadd_rn(x, x);
   const float n = rintf(y);
@@ -402,6 +422,15 @@ __device__ __forceinline__ float clamp_lb_ub(float x, float lo, float hi) {
   return x;
 }
 
+// The same in two instructions where neither a bound nor the position is a
+// negative zero (which lo = +0 would turn positive): NaN stays NaN.
+__device__ __forceinline__ float clamp_box(float x, float lo, float hi) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(lo));
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(y), "f"(hi));
+  return y;
+}
+
 // the velocity update of src/kernels.jl:2-9 in Julia's broadcast order:
 // ((w*v) + ((c1*r1)*(p-x))) + ((c2*r2)*(g-x))
 __device__ __forceinline__ float velocity(float x, float v, float p, float g, float w, float c1,
@@ -441,8 +470,9 @@ __device__ __forceinline__ float prm(const ObjParams& o, int k, float dflt) {
 }
 
 // Streaming accumulator over dims d = 0..D-1 (separable and chained
-// objectives).  add(d, x) must be called in increasing d.
-template <int OBJ>
+// objectives).  add(d, x) must be called in increasing d.  BOX: the cosines'
+// arguments are below 2^126 (box_cosines), cos2pi_box takes them.
+template <int OBJ, bool BOX = false>
 struct Acc {
   float s1 = 0.0f, s2 = 0.0f, prev = 0.0f;
   __device__ __forceinline__ void add(const ObjParams& o, int d, float x) {
@@ -457,10 +487,11 @@ struct Acc {
       }
       prev = x;
     } else if constexpr (OBJ == kRastrigin) {
-      s1 = __fadd_rn(s1, __fsub_rn(__fmul_rn(x, x), __fmul_rn(prm(o, 0, 10.0f), cos2pi(x))));
+      s1 = __fadd_rn(s1, __fsub_rn(__fmul_rn(x, x), __fmul_rn(prm(o, 0, 10.0f), BOX ? cos2pi_box(x) : cos2pi(x))));
     } else if constexpr (OBJ == kAckley) {
+      const float kx = __fmul_rn(prm(o, 2, 1.0f), x);
       s1 = __fadd_rn(s1, __fmul_rn(x, x));
-      s2 = __fadd_rn(s2, cos2pi(__fmul_rn(prm(o, 2, 1.0f), x)));
+      s2 = __fadd_rn(s2, BOX ? cos2pi_box(kx) : cos2pi(kx));
     } else if constexpr (OBJ == kShiftedSphere) {
       const float t = __fsub_rn(x, prm(o, d, 0.0f));  // test/constraints.jl:7
       s1 = __fadd_rn(s1, __fmul_rn(t, t));

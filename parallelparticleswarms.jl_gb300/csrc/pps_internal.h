@@ -83,6 +83,7 @@ int launch_async(pps_swarm* s, int iters, float c1, float c2, int* lanes_out);
 int launch_eval(const ObjParams& op, const ObjData& od, int objective, const float* x, int64_t npts,
                 int64_t stride, float* f, cudaStream_t stream);
 int async_lanes(int dim, int* slice);
+bool pair_form(const pps_swarm* s, float c1, float c2);  // whether the arithmetic of pps_pair.cuh is exact for a run
 int sync_grid(pps_swarm* s);
 // the TMA-staged step (pps_sync_bulk.cu): resident blocks per SM where it
 // applies (0 where it does not), resolved outside any stream capture; the
