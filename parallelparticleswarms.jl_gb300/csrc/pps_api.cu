@@ -525,10 +525,10 @@ static int run_steps(pps_swarm* s, int32_t maxiters, float c1, float c2, uint32_
 }
 
 // whether a run of this swarm keeps its state on chip (pps_resident.cu):
-// the swarm fits, its coefficients scale exactly (coef_scales), and the
+// the swarm fits, the pair arithmetic is exact for it (pair_form), and the
 // TMA-staged step kernel has not been asked for
 static bool resident_applies(const pps_swarm* s, float c1, float c2, ResidentPlan* plan) {
-  if (s->shard || !s->owns_memory || !coef_scales(c1) || !coef_scales(c2)) return false;
+  if (s->shard || !s->owns_memory || !pair_form(s, c1, c2)) return false;
   if (sync_bulk_requested()) return false;
   if (!resident_plan(s->objective, s->dv.dim, s->dv.n, s->dv.ncons, s->sm_count, plan)) return false;
   return plan->blocks == 1 || s->xch_dev;

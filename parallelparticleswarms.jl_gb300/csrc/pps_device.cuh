@@ -57,6 +57,10 @@ enum Objective : int {
   kBoundaryQuadratic = 20,
 };
 
+// a user objective (compiled by NVRTC with its source): f and, when the source
+// defines PPS_HAS_GRADIENT, pps_gradient(x, dim, p, data, ndata, g) returning f
+constexpr int kUserObjective = 255;
+
 // ---------------------------------------------------------------- Philox
 struct Rand4 {
   uint32_t a, b, c, d;

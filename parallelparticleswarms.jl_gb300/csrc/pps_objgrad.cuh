@@ -15,10 +15,6 @@ namespace pps {
 // arrays of the caller stay in registers.
 #define PPS_FOR_D(d) _Pragma("unroll") for (int d = 0; d < MAXD; ++d) if (d < D)
 
-// a user objective (compiled by NVRTC with its source): f and, when the source
-// defines PPS_HAS_GRADIENT, pps_gradient(x, dim, p, data, ndata, g) returning f
-constexpr int kUserObjective = 255;
-
 template <int OBJ, int MAXD>
 __device__ __forceinline__ float obj_value(const ObjParams& op, const float (&x)[MAXD], int D) {
 #ifdef PPS_USER_SOURCE

@@ -3,8 +3,11 @@
 //
 // Measured on a GB300, us an iteration, one launch per iteration -> resident:
 // Rosenbrock 1000 x 3 7.2 -> 1.7, Rastrigin 10000 x 10 9.4 -> 2.3, Ackley
-// 20011 x 30 16.2 -> 4.4, Rosenbrock 65536 x 10 9.4 -> 4.0, sphere 100003 x 20
-// 18.2 -> 5.9, Rastrigin 10000 x 100 36.1 -> 5.5, 250000 x 10 19.6 -> 9.6.  The
+// 20011 x 30 16.2 -> 4.4, Rosenbrock 65536 x 10 9.4 -> 3.9, sphere 100003 x 20
+// 18.2 -> 5.5, Rastrigin 10000 x 100 36.1 -> 5.5, 250000 x 10 19.6 -> 8.8,
+// 20011 x 128 45.5 -> 14.7 (the pair arithmetic of pps_pair.cuh took the last
+// three large ones from 5.9, 9.6 and 16.4; the small ones wait for the
+// exchange, 2100 cycles of 3700 at 1000 x 3, 3300 of 9100 at 20011 x 30).  The
 // line is the shared memory of all SMs (about 2.8 M coordinates of 12 bytes,
 // 2.1 M with the moved terms): beyond it the state has to stream from L2 or
 // memory each iteration, which k_sync_step does.
@@ -22,6 +25,8 @@ __global__ void __launch_bounds__(kResidentMaxThreads, 1)
 // polls of one word before a wait gives up: each is at least an L2 round trip
 // (several hundred cycles), so seconds -- no exchange takes milliseconds
 constexpr unsigned int kResidentPollLimit = 1u << 23;
+// a user objective may take its own time, and unevenly: minutes
+constexpr unsigned int kResidentUserPollLimit = 1u << 29;
 constexpr size_t kResidentSmem = 227u << 10;  // a block's shared memory, static part included
 constexpr size_t kResidentStatic = 2048;
 constexpr int kResidentMaxDim = 1024;  // g and bounds of more dims crowd the state out
@@ -41,24 +46,26 @@ size_t resident_exchange_bytes(int objective, int dim, int64_t n, int ncons, int
 static bool resident_fit(int objective, int dim, int64_t n, bool cons, int blocks, ResidentPlan* p) {
   const int64_t chunk = (n + blocks - 1) / blocks;
   const int np = (dim + 1) / 2;
+  const int most = is_user(objective) ? kResidentUserThreads : kResidentMaxThreads;
   if (chunk > (1 << 20)) return false;
-  int groups = (int)(kResidentMaxThreads / chunk);
+  int groups = (int)(most / chunk);
   if (groups > np) groups = np;
   if (groups > 1) groups = (np + (np + groups - 1) / groups - 1) / ((np + groups - 1) / groups);  // even shares
   bool split = cons || groups > 1;
   if (!cons && split && resident_smem(dim, (int)chunk, terms_moved(objective)) + kResidentStatic > kResidentSmem) {
     split = false;  // no room for the terms: one thread walks all dims
   }
+  split = split || is_user(objective);
   if (groups < 1 || !split) groups = 1;
-  p->smem = resident_smem(dim, (int)chunk, split && terms_moved(objective));
-  if (p->smem + kResidentStatic > kResidentSmem) return false;
   p->split = split;
   p->groups = groups;
   p->chunk = (int)chunk;
   p->blocks = (int)((n + chunk - 1) / chunk);
   const int64_t want = groups > 1 ? chunk * groups : chunk;
-  const int64_t rounds = (want + kResidentMaxThreads - 1) / kResidentMaxThreads;
+  const int64_t rounds = (want + most - 1) / most;
   p->threads = (int)(((want + rounds - 1) / rounds + 31) / 32 * 32);
+  p->smem = resident_smem(dim, (int)chunk, split && terms_moved(objective));
+  if (p->smem + kResidentStatic > kResidentSmem) return false;
   return true;
 }
 
@@ -66,7 +73,8 @@ bool resident_plan(int objective, int dim, int64_t n, int ncons, int sm_count, R
   switch (objective) {
     case kSphere: case kRosenbrock: case kRastrigin: case kAckley: case kShiftedSphere: case kBeale: case kBooth:
     case kHimmelblau: case kQuadratic: case kBoundaryQuadratic: break;
-    default: return false;
+    default:
+      if (!is_user(objective)) return false;
   }
   if (dim > kResidentMaxDim || n < 1 || sm_count < 1) return false;
   // Blocks: one while the iteration is shorter than an exchange between
@@ -78,14 +86,15 @@ bool resident_plan(int objective, int dim, int64_t n, int ncons, int sm_count, R
   const int64_t coords = n * (int64_t)((dim + 1) / 2 * 2);
   int64_t blocks = coords <= kResidentOneBlock ? 1 : coords / kResidentCoords;
   if (coords > kResidentOneBlock && blocks < kResidentMinBlocks) blocks = kResidentMinBlocks;
+  // a user objective's own cost is unknown: spread from a warp of particles a block
+  if (is_user(objective)) blocks = (n + 31) / 32;
   if (blocks > sm_count) blocks = sm_count;
   if (blocks > n) blocks = n;
   return resident_fit(objective, dim, n, ncons > 0, (int)blocks, p) ||
          resident_fit(objective, dim, n, ncons > 0, sm_count, p);
 }
 
-template <typename K>
-static int launch_one(K kernel, pps_swarm* s, const ResidentPlan& p, const PhiloxKeys& keys, const ResidentArgs& a,
+static int launch_one(const void* kernel, pps_swarm* s, const ResidentPlan& p, PhiloxKeys keys, ResidentArgs a,
                       bool* taken) {
   if (p.smem + kResidentStatic > (48u << 10))
     PPS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -103,23 +112,24 @@ static int launch_one(K kernel, pps_swarm* s, const ResidentPlan& p, const Philo
     at[0].val.cooperative = 1;
     cfg.numAttrs = 1;
   }
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, s->dv, s->op, keys, a);
+  void* args[] = {&s->dv, &s->op, &keys, &a};
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
   if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device reports: step by step instead
     cudaGetLastError();
     return PPS_OK;
   }
-  if (e != cudaSuccess) return cuda_error(e, "cudaLaunchKernelEx(k_resident)");
+  if (e != cudaSuccess) return cuda_error(e, "cudaLaunchKernelExC(k_resident)");
   *taken = true;
   return PPS_OK;
 }
 
 template <int OBJ>
 static int launch_obj(pps_swarm* s, const ResidentPlan& p, const PhiloxKeys& keys, const ResidentArgs& a, bool* taken) {
-  if (s->dv.ncons > 0) return launch_one(k_resident<OBJ, true, true>, s, p, keys, a, taken);
+  if (s->dv.ncons > 0) return launch_one(reinterpret_cast<const void*>(k_resident<OBJ, true, true>), s, p, keys, a, taken);
   if constexpr (OBJ < kBeale) {
-    if (p.split) return launch_one(k_resident<OBJ, true, false>, s, p, keys, a, taken);
+    if (p.split) return launch_one(reinterpret_cast<const void*>(k_resident<OBJ, true, false>), s, p, keys, a, taken);
   }
-  return launch_one(k_resident<OBJ, false, false>, s, p, keys, a, taken);
+  return launch_one(reinterpret_cast<const void*>(k_resident<OBJ, false, false>), s, p, keys, a, taken);
 }
 
 int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w, float wdamp, float c1, float c2,
@@ -137,9 +147,21 @@ int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w,
   a.from_position = from_position;
   a.seq0 = s->xch_seq;
   a.poll_limit = kResidentPollLimit;
+  a.one = 1.0f;
   a.xch = s->xch_dev;
   const PhiloxKeys keys = philox_round_keys(s->seed);
   int rc;
+  if (is_user(s->objective)) {
+    const void* kernel = nullptr;
+    if ((rc = user_resident_kernel(s->objective, &kernel))) return rc;
+    cudaFuncAttributes fa;
+    PPS_CUDA(cudaFuncGetAttributes(&fa, kernel));
+    if (fa.sharedSizeBytes > kResidentStatic) return PPS_OK;  // the source's own shared memory leaves no room
+    a.poll_limit = kResidentUserPollLimit;
+    rc = launch_one(kernel, s, p, keys, a, taken);
+    if (*taken) s->xch_seq += (uint32_t)iters;
+    return rc;
+  }
   switch (s->objective) {
     case kSphere: rc = launch_obj<kSphere>(s, p, keys, a, taken); break;
     case kRosenbrock: rc = launch_obj<kRosenbrock>(s, p, keys, a, taken); break;

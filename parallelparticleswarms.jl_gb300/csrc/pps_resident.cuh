@@ -24,9 +24,13 @@
 //     posts.  Two buffers alternate: a block can only be one exchange ahead of
 //     another, since it needs the other's post to go on.  The grid is a
 //     cooperative launch, so every block is resident.
+// A user objective (kUserObjective, compiled by NVRTC) reads the new position
+// back through its accessor, so its state lies at [dim][particle]; the
+// read-back is from shared memory instead of L2.
 // The wait for a post is bounded (poll_limit polls); a wait that gives up sets
 // IterState::status bit 3 and the block leaves the loop.
 #pragma once
+#include "pps_pair.cuh"
 #include "pps_publish.cuh"
 
 namespace pps {
@@ -41,6 +45,7 @@ struct ResidentArgs {
   int from_position;
   uint32_t seq0;      // sequence number before the first exchange
   unsigned int poll_limit;
+  float one;          // 1.0f (pps_pair.cuh)
   unsigned long long* xch;  // exchange of a grid of several blocks: two buffers of resident_words
 };
 
@@ -49,6 +54,7 @@ template <int OBJ>
 constexpr bool kTermsMoved = OBJ == kRastrigin || OBJ == kAckley;
 
 constexpr int kResidentMaxThreads = 1024;
+constexpr int kResidentUserThreads = 512;  // 128 registers for a user objective
 
 // shared memory of a block: bounds (float4 per pair), g (float2 per pair),
 // x, v, pbest (float2 per pair and particle), the moved terms, pcost, flags
@@ -75,14 +81,6 @@ __device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k)
   const uint32_t m = __reduce_min_sync(0xffffffffu, hi);
   const uint32_t i = __reduce_min_sync(0xffffffffu, hi == m ? lo : 0xffffffffu);
   return ((unsigned long long)m << 32) | (unsigned long long)i;
-}
-
-// one coordinate's term of an objective that is a sum of them (kTermsMoved)
-template <int OBJ>
-__device__ __forceinline__ float moved_term(const ObjParams& op, float x) {
-  if constexpr (OBJ == kRastrigin) return __fsub_rn(__fmul_rn(x, x), __fmul_rn(prm(op, 0, 10.0f), cos2pi(x)));
-  if constexpr (OBJ == kAckley) return cos2pi(__fmul_rn(prm(op, 2, 1.0f), x));
-  return 0.0f;
 }
 
 __device__ __forceinline__ void post_word(unsigned long long* p, unsigned long long v) {
@@ -139,10 +137,49 @@ __device__ __forceinline__ unsigned long long await_keys(const unsigned long lon
   return warp_min_key(best);
 }
 
+// the objective of a user source at particle p, its position in rows
+#ifdef PPS_USER_SOURCE
+__device__ __forceinline__ float user_value(const float2* X, int p, int chunk, int D, const float* prm8,
+                                            const ObjParams& op) {
+  return pps_objective(pps_point{reinterpret_cast<const float*>(X) + p, chunk}, D, prm8, op.data, op.ndata);
+}
+#else
+__device__ __forceinline__ float user_value(const float2*, int, int, int, const float*, const ObjParams&) {
+  return 0.0f;
+}
+#endif
+
+// a pair's x, v or pbest: float2 at [pair][particle], or ROWS: floats at [dim][particle]
+template <bool ROWS>
+__device__ __forceinline__ float2 pair_get(const float2* A, int j, int p, int chunk) {
+  if constexpr (ROWS) {
+    const float* f = reinterpret_cast<const float*>(A) + 2 * j * chunk + p;
+    return make_float2(f[0], f[chunk]);
+  } else {
+    return A[j * chunk + p];
+  }
+}
+template <bool ROWS>
+__device__ __forceinline__ void pair_put(float2* A, int j, int p, int chunk, float2 v) {
+  if constexpr (ROWS) {
+    float* f = reinterpret_cast<float*>(A) + 2 * j * chunk + p;
+    f[0] = v.x;
+    f[chunk] = v.y;
+  } else {
+    A[j * chunk + p] = v;
+  }
+}
+template <bool ROWS>
+__device__ __forceinline__ float coord_get(const float2* A, int d, int p, int chunk) {
+  return reinterpret_cast<const float*>(A)[ROWS ? d * chunk + p : 2 * ((d >> 1) * chunk + p) + (d & 1)];
+}
+
+// `prm8`: a user objective's 8 parameters in shared memory
 template <int OBJ, bool SPLIT, bool CONS>
 __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams& op, const PhiloxKeys& keys,
-                                             const ResidentArgs& a) {
-  static_assert(SPLIT || !CONS, "the constrained form sums in its own phase");
+                                             const ResidentArgs& a, const float* prm8 = nullptr) {
+  static_assert(SPLIT || !(CONS || OBJ == kUserObjective), "constraints and user objectives are summed in a phase of their own");
+  constexpr bool ROWS = OBJ == kUserObjective;
   extern __shared__ __align__(16) float rsm[];
   __shared__ unsigned long long red[2][32];
   __shared__ unsigned long long win_s;
@@ -178,9 +215,9 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     for (int j = warp; j < np; j += nw) {
       const int64_t o = (int64_t)(2 * j) * s.npad + first + p;
       const bool two = 2 * j + 1 < D;
-      X[j * chunk + p] = make_float2(s.X[o], two ? s.X[o + s.npad] : 0.0f);
-      V[j * chunk + p] = make_float2(s.V[o], two ? s.V[o + s.npad] : 0.0f);
-      P[j * chunk + p] = make_float2(s.P[o], two ? s.P[o + s.npad] : 0.0f);
+      pair_put<ROWS>(X, j, p, chunk, make_float2(s.X[o], two ? s.X[o + s.npad] : 0.0f));
+      pair_put<ROWS>(V, j, p, chunk, make_float2(s.V[o], two ? s.V[o + s.npad] : 0.0f));
+      pair_put<ROWS>(P, j, p, chunk, make_float2(s.P[o], two ? s.P[o + s.npad] : 0.0f));
     }
   }
   __syncthreads();
@@ -192,6 +229,8 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     p0 = g0 < G ? tid - g0 * chunk : cnt;
   }
   const int stride = (SPLIT && G > 1) ? chunk : T;  // one particle per thread when pairs are shared
+  using namespace pair32;
+  const float2 c1 = dup(a.c1s), c2 = dup(a.c2s), one2 = dup(a.one), mone2 = dup(-a.one);
   float w = a.w0;
   unsigned long long win = ~0ull, prev = ~0ull;
   bool have_prev = false;
@@ -218,29 +257,36 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
       PhiloxIteration pi;
       pi.start(pp, t, keys);
       const bool fl = flag[p] != 0;
-      Acc<OBJ> acc;
+      const float2 w2 = dup(w);
+      Acc<OBJ, true> acc;
 #pragma unroll 1
       for (int j = g0; j < np; j += G) {
         const Rand4 r = pi.draw((uint32_t)j, keys);
-        const int o = j * chunk + p;
-        float2 x = X[o], v = V[o], q = P[o];
+        const float2 x = pair_get<ROWS>(X, j, p, chunk);
+        float2 q = pair_get<ROWS>(P, j, p, chunk);
         if (fl) {  // the personal-best copy deferred from the last iteration
           q = x;
-          P[o] = q;
+          pair_put<ROWS>(P, j, p, chunk, q);
         }
-        const float2 gd = g2[j];
         const float4 b = bnd[j];
-        v.x = velocity24(x.x, v.x, q.x, gd.x, w, a.c1s, a.c2s, r.a, r.b);
-        v.y = velocity24(x.y, v.y, q.y, gd.y, w, a.c1s, a.c2s, r.c, r.d);
-        x.x = clamp_lb_ub(__fadd_rn(x.x, v.x), b.x, b.y);
-        x.y = clamp_lb_ub(__fadd_rn(x.y, v.y), b.z, b.w);
-        X[o] = x;
-        V[o] = v;
-        if constexpr (!SPLIT) {
-          acc.add(op, 2 * j, x.x);
-          if (2 * j + 1 < D) acc.add(op, 2 * j + 1, x.y);
+        const float2 v =
+            velocity24x2(x, pair_get<ROWS>(V, j, p, chunk), q, g2[j], w2, c1, c2, r, one2, mone2);
+        float2 y = add(x, v);
+        y.x = clamp_box(y.x, b.x, b.y);
+        y.y = clamp_box(y.y, b.z, b.w);
+        pair_put<ROWS>(X, j, p, chunk, y);
+        pair_put<ROWS>(V, j, p, chunk, v);
+        const bool two = 2 * j + 1 < D;
+        if constexpr (ROWS) {
         } else if constexpr (TERMS) {
-          TM[o] = make_float2(moved_term<OBJ>(op, x.x), moved_term<OBJ>(op, x.y));
+          TM[j * chunk + p] = moved_terms<OBJ>(op, y, mone2);
+        } else if constexpr (!SPLIT && kTermsMoved<OBJ>) {
+          const float2 m = moved_terms<OBJ>(op, y, mone2);
+          add_term<OBJ>(acc, y.x, m.x);
+          if (two) add_term<OBJ>(acc, y.y, m.y);
+        } else if constexpr (!SPLIT) {
+          acc.add(op, 2 * j, y.x);
+          if (two) acc.add(op, 2 * j + 1, y.y);
         }
       }
       if constexpr (!SPLIT) settle(p, finalize<OBJ>(op, acc.s1, acc.s2));
@@ -249,33 +295,37 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     if constexpr (SPLIT) {
       __syncthreads();
       for (int p = tid; p < cnt; p += T) {
-        Acc<OBJ> acc;
+        Acc<OBJ, true> acc;
         ConsAcc ca;
         if constexpr (CONS) ca.start(s.cons, s.ncons, D);
         auto add = [&](int d, float x, float term) {
-          if constexpr (OBJ == kRastrigin) {
-            acc.s1 = __fadd_rn(acc.s1, term);
-          } else if constexpr (OBJ == kAckley) {
-            acc.s1 = __fadd_rn(acc.s1, __fmul_rn(x, x));
-            acc.s2 = __fadd_rn(acc.s2, term);
-          } else {
+          if constexpr (TERMS) {
+            add_term<OBJ>(acc, x, term);
+          } else if constexpr (!ROWS) {
             acc.add(op, d, x);
           }
           if constexpr (CONS) ca.add(s.cons, s.ncons, D, d, x);
         };
         const int full = D >> 1;
+        if (!ROWS || s.ncons > 0) {  // a user objective reads its position itself
 #pragma unroll 4
-        for (int j = 0; j < full; ++j) {
-          const float2 x = X[j * chunk + p], m = TERMS ? TM[j * chunk + p] : x;
-          add(2 * j, x.x, m.x);
-          add(2 * j + 1, x.y, m.y);
+          for (int j = 0; j < full; ++j) {
+            const float2 x = pair_get<ROWS>(X, j, p, chunk), m = TERMS ? TM[j * chunk + p] : x;
+            add(2 * j, x.x, m.x);
+            add(2 * j + 1, x.y, m.y);
+          }
+          if (D & 1) {
+            const float2 x = pair_get<ROWS>(X, full, p, chunk), m = TERMS ? TM[full * chunk + p] : x;
+            add(D - 1, x.x, m.x);
+          }
         }
-        if (D & 1) {
-          const float2 x = X[full * chunk + p], m = TERMS ? TM[full * chunk + p] : x;
-          add(D - 1, x.x, m.x);
+        float c;
+        if constexpr (ROWS) {
+          c = user_value(X, p, chunk, D, prm8, op);
+        } else {
+          c = finalize<OBJ>(op, acc.s1, acc.s2);
         }
-        float c = finalize<OBJ>(op, acc.s1, acc.s2);
-        if constexpr (CONS) c = __fadd_rn(c, penalty(ca, s.ncons, __uint2float_rn((uint32_t)(first + p) + 2u)));
+        if (CONS && (!ROWS || s.ncons > 0)) c = __fadd_rn(c, penalty(ca, s.ncons, __uint2float_rn((uint32_t)(first + p) + 2u)));
         settle(p, c);
       }
     }
@@ -286,8 +336,8 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     const unsigned long long mine = warp_min_key(lane < nw ? red[par][lane] : ~0ull);
     const int lp = (int)((int64_t)(uint32_t)mine - first);  // its particle (meaningless when mine is ~0)
     const bool none = mine == ~0ull;
-    const float* src = nullptr;  // its vector: the position if it improved just now, else the personal best
-    if (!none) src = reinterpret_cast<const float*>((a.from_position || flag[lp]) ? X : P);
+    const float2* src = nullptr;  // its vector: the position if it improved just now, else the personal best
+    if (!none) src = (a.from_position || flag[lp]) ? X : P;
     // ---- agree on the global best
     const uint32_t seq = a.seq0 + 1u + (uint32_t)it;
     const int nb = (int)gridDim.x;
@@ -295,7 +345,7 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     unsigned long long* vw = kw + 2 * (size_t)nb;                          // vectors
     if (nb == 1) {
       win = mine;
-      for (int d = tid; d < D; d += T) gs[d] = src[2 * ((d >> 1) * chunk + lp) + (d & 1)];
+      for (int d = tid; d < D; d += T) gs[d] = coord_get<ROWS>(src, d, lp, chunk);
     } else {
       if (tid == 0) {
         post_word(kw + 2 * (size_t)blockIdx.x, resident_word((uint32_t)(mine >> 32), seq));
@@ -304,7 +354,7 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
       if (!none)
         for (int d = tid; d < D; d += T)
           post_word(vw + (size_t)blockIdx.x * D + d,
-                    resident_word(__float_as_uint(src[2 * ((d >> 1) * chunk + lp) + (d & 1)]), seq));
+                    resident_word(__float_as_uint(coord_get<ROWS>(src, d, lp, chunk)), seq));
     }
     if (nb > 1 && warp == 0) {
       bool ok = true;
@@ -343,8 +393,8 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     const bool fl = flag[p] != 0;
     for (int j = warp; j < np; j += nw) {
       const int64_t o = (int64_t)(2 * j) * s.npad + first + p;
-      const float2 x = X[j * chunk + p], v = V[j * chunk + p];
-      const float2 q = fl ? x : P[j * chunk + p];
+      const float2 x = pair_get<ROWS>(X, j, p, chunk), v = pair_get<ROWS>(V, j, p, chunk);
+      const float2 q = fl ? x : pair_get<ROWS>(P, j, p, chunk);
       s.X[o] = x.x;
       s.V[o] = v.x;
       s.P[o] = q.x;

@@ -95,9 +95,10 @@ struct UserObjective {
   std::atomic<bool> loaded{false};
   cudaLibrary_t lib = nullptr;
   cudaKernel_t k_init = nullptr, k_eval = nullptr;
-  cudaKernel_t k_step[3] = {};  // 1, 2, 4 particles per thread
+  cudaKernel_t k_step = nullptr;  // PPS_USER_PPT particles per thread
   cudaKernel_t k_step_cons = nullptr;
   cudaKernel_t k_async = nullptr;
+  cudaKernel_t k_resident = nullptr;
   // HybridPSO's local stage, when the source has a gradient (else NULL)
   cudaKernel_t k_lbfgs16 = nullptr, k_lbfgs64 = nullptr, k_broyden16 = nullptr;
 };
@@ -128,6 +129,17 @@ int current_arch() {
   return major * 10 + minor;
 }
 
+// particles per thread of the unconstrained step kernel; PPS_USER_PPT=1|2|4
+// overrides the default
+int user_step_ppt() {
+  static const int ppt = [] {
+    const char* e = getenv("PPS_USER_PPT");
+    const int v = e ? atoi(e) : 2;
+    return (v == 1 || v == 2 || v == 4) ? v : 2;
+  }();
+  return ppt;
+}
+
 int compile(const std::string& user, int arch, std::vector<char>* out) {
   const NvrtcApi& api = nvrtc();
   if (!api.handle) return set_error(PPS_ENOTSUP, "user objectives need NVRTC: %s", api.why.c_str());
@@ -149,6 +161,8 @@ int compile(const std::string& user, int arch, std::vector<char>* out) {
   }
   std::vector<const char*> opts = {target.c_str(), "-std=c++17", "--fmad=false", "-lineinfo"};
   if (!minblocks.empty()) opts.push_back(minblocks.c_str());
+  const std::string ppt = "-DPPS_USER_PPT=" + std::to_string(user_step_ppt());
+  opts.push_back(ppt.c_str());
   r = api.compile(prog, (int)opts.size(), opts.data());
   if (r != NVRTC_SUCCESS) {
     size_t n = 0;
@@ -179,11 +193,10 @@ int ensure_loaded(UserObjective* u) {
   if (u->loaded.load(std::memory_order_relaxed)) return PPS_OK;
   PPS_CUDA(cudaLibraryLoadData(&u->lib, u->cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
   PPS_CUDA(cudaLibraryGetKernel(&u->k_init, u->lib, "pps_user_init"));
-  PPS_CUDA(cudaLibraryGetKernel(&u->k_step[0], u->lib, "pps_user_step1"));
-  PPS_CUDA(cudaLibraryGetKernel(&u->k_step[1], u->lib, "pps_user_step2"));
-  PPS_CUDA(cudaLibraryGetKernel(&u->k_step[2], u->lib, "pps_user_step4"));
+  PPS_CUDA(cudaLibraryGetKernel(&u->k_step, u->lib, "pps_user_step"));
   PPS_CUDA(cudaLibraryGetKernel(&u->k_step_cons, u->lib, "pps_user_step_cons"));
   PPS_CUDA(cudaLibraryGetKernel(&u->k_async, u->lib, "pps_user_async"));
+  PPS_CUDA(cudaLibraryGetKernel(&u->k_resident, u->lib, "pps_user_resident"));
   if (cudaLibraryGetKernel(&u->k_lbfgs16, u->lib, "pps_user_lbfgs16") != cudaSuccess) {
     cudaGetLastError();  // no gradient in the source: no local stage
     u->k_lbfgs16 = nullptr;
@@ -208,17 +221,6 @@ UserObjective* loaded_or_error(int objective, int* rc) {
 
 constexpr int kUserThreads = 256;
 
-// particles per thread of the unconstrained step kernel; PPS_USER_PPT=1|2|4
-// overrides the default
-int user_step_ppt() {
-  static const int ppt = [] {
-    const char* e = getenv("PPS_USER_PPT");
-    const int v = e ? atoi(e) : 2;
-    return (v == 1 || v == 2 || v == 4) ? v : 2;
-  }();
-  return ppt;
-}
-
 }  // namespace
 
 bool is_user(int objective) { return lookup(objective) != nullptr; }
@@ -232,7 +234,7 @@ int user_prepare(pps_swarm* s) {
   const void* k = reinterpret_cast<const void*>(u->k_step_cons);
   if (s->dv.ncons == 0) {
     ppt = user_step_ppt();
-    k = reinterpret_cast<const void*>(u->k_step[ppt == 1 ? 0 : (ppt == 2 ? 1 : 2)]);
+    k = reinterpret_cast<const void*>(u->k_step);
   }
   const size_t smem = 3 * sizeof(float) * (size_t)s->dv.dim;
   // g, lb, ub in dynamic shared memory: beyond 40 kB (3414 dims) the kernel
@@ -274,6 +276,14 @@ int launch_user_step(pps_swarm* s, float c1, float c2) {
   void* args[] = {&s->dv, &s->op, &data, &ndata, &keys, &c1, &c2, &from_pos};
   PPS_CUDA(cudaLaunchKernel(s->user_step_kernel, dim3((unsigned)s->user_grid), dim3(kUserThreads), args,
                             3 * sizeof(float) * (size_t)s->dv.dim, s->stream));
+  return PPS_OK;
+}
+
+int user_resident_kernel(int objective, const void** kernel) {
+  int rc;
+  UserObjective* u = loaded_or_error(objective, &rc);
+  if (!u) return rc;
+  *kernel = reinterpret_cast<const void*>(u->k_resident);
   return PPS_OK;
 }
 

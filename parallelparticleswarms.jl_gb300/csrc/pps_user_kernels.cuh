@@ -16,6 +16,7 @@
 // problem carries constraints.
 #pragma once
 #include "pps_publish.cuh"
+#include "pps_resident.cuh"
 #include "pps_vec.cuh"
 
 // resident blocks each kernel is compiled for (register cap 65536 / (256 x
@@ -251,16 +252,15 @@ __device__ __forceinline__ void user_step(const SwarmDev& s, const ObjParams& op
 
 }  // namespace pps
 
-extern "C" __global__ void __launch_bounds__(pps::kUserThreads, PPS_USER_MB4)
-    pps_user_step1(pps::SwarmDev s, pps::ObjParams op, const float* data, long long ndata, pps::PhiloxKeys keys,
-                   float c1, float c2, int from_position) {
-  pps::user_step<1, false>(s, op, data, ndata, keys, c1, c2, from_position);
-}
-
-extern "C" __global__ void __launch_bounds__(pps::kUserThreads, PPS_USER_MB4)
-    pps_user_step2(pps::SwarmDev s, pps::ObjParams op, const float* data, long long ndata, pps::PhiloxKeys keys,
-                   float c1, float c2, int from_position) {
-  pps::user_step<2, false>(s, op, data, ndata, keys, c1, c2, from_position);
+// the unconstrained step with the particles per thread in use (PPS_USER_PPT,
+// 2 unless overridden): one instantiation, every source pays for its compilation
+#ifndef PPS_USER_PPT
+#define PPS_USER_PPT 2
+#endif
+extern "C" __global__ void __launch_bounds__(pps::kUserThreads, PPS_USER_PPT == 4 ? PPS_USER_MB2 : PPS_USER_MB4)
+    pps_user_step(pps::SwarmDev s, pps::ObjParams op, const float* data, long long ndata, pps::PhiloxKeys keys,
+                  float c1, float c2, int from_position) {
+  pps::user_step<PPS_USER_PPT, false>(s, op, data, ndata, keys, c1, c2, from_position);
 }
 
 // the constrained path: calc_penalty with iter = the 1-based particle index
@@ -271,10 +271,15 @@ extern "C" __global__ void __launch_bounds__(pps::kUserThreads, PPS_USER_MB4)
   pps::user_step<1, true>(s, op, data, ndata, keys, c1, c2, from_position);
 }
 
-extern "C" __global__ void __launch_bounds__(pps::kUserThreads, PPS_USER_MB2)
-    pps_user_step4(pps::SwarmDev s, pps::ObjParams op, const float* data, long long ndata, pps::PhiloxKeys keys,
-                   float c1, float c2, int from_position) {
-  pps::user_step<4, false>(s, op, data, ndata, keys, c1, c2, from_position);
+// A whole synchronous run with the state in shared memory (pps_resident.cuh),
+// with or without constraints and however many threads share a particle: one
+// instantiation, since every source pays for its compilation.
+extern "C" __global__ void __launch_bounds__(pps::kResidentUserThreads, 1)
+    pps_user_resident(pps::SwarmDev s, pps::ObjParams op, pps::PhiloxKeys keys, pps::ResidentArgs a) {
+  __shared__ float sp[8];
+  pps::user_params(sp, op);
+  __syncthreads();
+  pps::resident_run<pps::kUserObjective, true, true>(s, op, keys, a, sp);
 }
 
 // ParallelPSOKernel(global_update = false) for a user objective: the whole run

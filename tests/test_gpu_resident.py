@@ -113,3 +113,25 @@ def test_two_swarms_from_two_threads(pps, orc):
     for sw, ref in pairs:
         assert_state_equal(sw, ref, "100 iterations")
         sw.close()
+
+
+@pytest.mark.parametrize("D,n", [(1, 31), (3, 1000), (20, 4097), (33, 20000), (7, 200000)])
+@pytest.mark.parametrize("cons", [False, True])
+def test_user_objective_matches_the_registered_run(pps, D, n, cons):
+    """A source that spells Rastrigin, its position read back from shared memory, against the registered
+    kernel: one and several threads per particle, the last pair of an odd dim count, constraints."""
+    import user_sources as us
+    rows = np.stack([pps.quadratic_constraint(D, c=-2.0 * D, b=np.ones(D))]) if cons else None
+    lb, ub = np.full(D, -4.0, np.float32), np.full(D, 5.0, np.float32)
+    reg = pps.OptimizationProblem(pps.rastrigin, np.zeros(D, np.float32), [10.0], lb=lb, ub=ub, cons=rows)
+    usr = reg.remake(f=pps.cuda_objective(us.RASTRIGIN))
+    with pps.Swarm(reg, n, seed=8) as a, pps.Swarm(usr, n, seed=8) as b:
+        a.init()
+        b.init()
+        for k in (1, 2, 9):
+            a.sync_run(k)
+            b.sync_run(k)
+        sa, sb = a.state(), b.state()
+        for f in sa:
+            assert np.array_equal(sa[f], sb[f]), f
+        assert a.gbest()[1:] == b.gbest()[1:] and np.array_equal(a.gbest()[0], b.gbest()[0])
