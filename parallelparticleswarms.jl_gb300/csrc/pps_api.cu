@@ -168,11 +168,11 @@ static SwarmLayout swarm_layout(const pps_problem* prob, int64_t n, bool shard =
   L.oPc = take(sizeof(float) * L.npad);
   L.oC = take(sizeof(float) * L.npad);
   L.oF = take(L.npad);
+  L.oSt = take(sizeof(IterState));  // directly before g: one copy reads both
   L.oG = take(sizeof(float) * D);
-  L.oLb = take(sizeof(float) * D);
+  L.oLb = take(sizeof(float) * D);  // lb, ub, u0: one copy writes them
   L.oUb = take(sizeof(float) * D);
   L.oU0 = take(sizeof(float) * D);
-  L.oSt = take(sizeof(IterState));
   L.oData = take(sizeof(float) * (prob->data ? (size_t)prob->ndata : 0));
   L.mlp_samples = prob->objective == kMlp ? (int)(prob->ndata / 17) : 0;
   L.oMlpA = take(L.mlp_samples ? mlp_a_bytes(L.mlp_samples) : 0);
@@ -229,19 +229,18 @@ static int swarm_setup(pps_swarm* s, const pps_problem* prob, int64_t n, uint64_
   s->objective = prob->objective;
   s->seed = seed;
   s->flags = flags;
-  s->host_lb = static_cast<float*>(malloc(sizeof(float) * 3 * D));
+  const size_t row = (L.oUb - L.oLb) / sizeof(float);  // the device arrays' distance, so one copy serves
+  s->host_lb = static_cast<float*>(calloc(3 * row, sizeof(float)));
   if (!s->host_lb) return set_error(PPS_ENOMEM, "host allocation failed");
-  s->host_ub = s->host_lb + D;
-  s->host_u0 = s->host_lb + 2 * D;
+  s->host_ub = s->host_lb + row;
+  s->host_u0 = s->host_lb + 2 * row;
   for (int d = 0; d < D; ++d) {
     s->host_lb[d] = prob->lb ? prob->lb[d] : -INFINITY;
     s->host_ub[d] = prob->ub ? prob->ub[d] : INFINITY;
     s->host_u0[d] = prob->u0 ? prob->u0[d] : 0.0f;
   }
   PPS_CUDA(cudaMemsetAsync(b, 0, L.bytes + extra, s->stream));
-  PPS_CUDA(cudaMemcpyAsync(s->dv.lb, s->host_lb, sizeof(float) * D, cudaMemcpyHostToDevice, s->stream));
-  PPS_CUDA(cudaMemcpyAsync(s->dv.ub, s->host_ub, sizeof(float) * D, cudaMemcpyHostToDevice, s->stream));
-  PPS_CUDA(cudaMemcpyAsync(s->u0_dev, s->host_u0, sizeof(float) * D, cudaMemcpyHostToDevice, s->stream));
+  PPS_CUDA(cudaMemcpyAsync(s->dv.lb, s->host_lb, sizeof(float) * (2 * row + D), cudaMemcpyHostToDevice, s->stream));
   if (prob->data && prob->ndata > 0)
     PPS_CUDA(cudaMemcpyAsync(s->data_dev, prob->data, sizeof(float) * (size_t)prob->ndata, cudaMemcpyHostToDevice,
                              s->stream));
@@ -299,6 +298,9 @@ extern "C" {
 
 namespace pps {
 
+// Swarms up to this size take their block from the memory pool.
+constexpr size_t kPooledBlock = (size_t)32 << 20;
+
 // pps_swarm_create, and for a shard (nglobal > 0) pps_shard_create: the
 // swarm holds n particles, particles first .. first + n - 1 of nglobal
 int swarm_create(const pps_problem* prob, int64_t n, uint64_t seed, uint32_t flags, int64_t first,
@@ -320,19 +322,22 @@ int swarm_create(const pps_problem* prob, int64_t n, uint64_t seed, uint32_t fla
   const bool shard = nglobal > 0;
   const SwarmLayout L = swarm_layout(prob, n, shard);
   const size_t xch = shard ? 0 : resident_exchange_bytes(prob->objective, prob->dim, n, prob->ncons, s->sm_count);
-  cudaError_t e = cudaMalloc(&s->block, L.bytes + xch);
-  if (e != cudaSuccess) {
-    delete s;
-    return cuda_error(e, "cudaMalloc(swarm state)");
-  }
+  cudaError_t e;
   rc = PPS_OK;
   do {
-    if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess) {
+    PoolStream ps;
+    if ((e = pool_stream_get(s->device, &ps)) != cudaSuccess) {
       rc = cuda_error(e, "cudaStreamCreate");
       break;
     }
-    if ((e = cudaEventCreate(&s->ev0)) != cudaSuccess || (e = cudaEventCreate(&s->ev1)) != cudaSuccess) {
-      rc = cuda_error(e, "cudaEventCreate");
+    s->stream = ps.stream;
+    s->ev0 = ps.ev0;
+    s->ev1 = ps.ev1;
+    s->pooled = L.bytes + xch <= kPooledBlock;
+    e = s->pooled ? pool_alloc(s->device, &s->block, L.bytes + xch, s->stream) : cudaMalloc(&s->block, L.bytes + xch);
+    if (e != cudaSuccess) {
+      s->block = nullptr;
+      rc = cuda_error(e, "cudaMalloc(swarm state)");
       break;
     }
     if ((rc = swarm_setup(s, prob, n, seed, flags, static_cast<char*>(s->block), L, xch))) break;
@@ -372,11 +377,15 @@ int pps_swarm_destroy(pps_swarm* s) {
   if (dev != s->device) cudaSetDevice(s->device);
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->graph) cudaGraphExecDestroy(s->graph);
-  if (s->ev0) cudaEventDestroy(s->ev0);
-  if (s->ev1) cudaEventDestroy(s->ev1);
-  if (s->stream) cudaStreamDestroy(s->stream);
-  if (s->block) cudaFree(s->block);
+  if (s->block) {
+    if (s->pooled)
+      cudaFreeAsync(s->block, s->stream);
+    else
+      cudaFree(s->block);
+  }
   if (s->local_block) cudaFree(s->local_block);
+  PoolStream ps{s->stream, s->ev0, s->ev1};
+  pool_stream_put(s->device, &ps);
   free(s->host_lb);
   if (dev >= 0 && dev != s->device) cudaSetDevice(dev);
   delete s;
@@ -608,10 +617,15 @@ int pps_get_gbest(pps_swarm* s, float* u, float* cost, int64_t* idx) {
   if (!s->initialized) return set_error(PPS_EINVAL, "swarm is not initialised");
   int rc = use_device(s);
   if (rc) return rc;
-  IterState st;
-  PPS_CUDA(cudaMemcpyAsync(&st, s->dv.st, sizeof(st), cudaMemcpyDeviceToHost, s->stream));
-  if (u) PPS_CUDA(cudaMemcpyAsync(u, s->dv.g, sizeof(float) * s->dv.dim, cudaMemcpyDeviceToHost, s->stream));
+  // the state and, behind it in the layout, g
+  const size_t at = (size_t)(reinterpret_cast<char*>(s->dv.g) - reinterpret_cast<char*>(s->dv.st));
+  const size_t vec = u ? sizeof(float) * (size_t)s->dv.dim : 0;
+  std::vector<char> host(at + vec);
+  PPS_CUDA(cudaMemcpyAsync(host.data(), s->dv.st, host.size(), cudaMemcpyDeviceToHost, s->stream));
   PPS_CUDA(cudaStreamSynchronize(s->stream));
+  IterState st;
+  memcpy(&st, host.data(), sizeof(st));
+  if (u) memcpy(u, host.data() + at, vec);
   if (cost) *cost = st.gcost;
   if (idx) *idx = (int64_t)st.gidx;
   return PPS_OK;
@@ -748,8 +762,7 @@ int pps_set_state(pps_swarm* s, int32_t field, const float* in) {
 // swarm may be re-run or destroyed while the snapshot lives.
 struct pps_field_copy {
   int device = 0;
-  cudaStream_t stream = nullptr;
-  cudaEvent_t ready = nullptr;
+  pps::PoolStream ps;  // its stream reads and frees the copy, ev0 marks it complete
   float* dev = nullptr;
   int rows = 0;
   int64_t n = 0;
@@ -768,13 +781,12 @@ int pps_field_copy_create(pps_swarm* s, int32_t field, pps_field_copy** out) {
   c->rows = rows;
   c->n = s->dv.n;
   const size_t w = sizeof(float) * (size_t)s->dv.n;
-  cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ready, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&c->dev), w * (size_t)rows, s->stream);
+  cudaError_t e = pool_stream_get(c->device, &c->ps);
+  if (e == cudaSuccess) e = pool_alloc(c->device, reinterpret_cast<void**>(&c->dev), w * (size_t)rows, s->stream);
   if (e == cudaSuccess)
     e = cudaMemcpy2DAsync(c->dev, w, src, sizeof(float) * (size_t)s->dv.npad, w, (size_t)rows,
                           cudaMemcpyDeviceToDevice, s->stream);
-  if (e == cudaSuccess) e = cudaEventRecord(c->ready, s->stream);
+  if (e == cudaSuccess) e = cudaEventRecord(c->ps.ev0, s->stream);
   if (e != cudaSuccess) {
     pps_field_copy_destroy(c);
     return cuda_error(e, "pps_field_copy_create");
@@ -786,9 +798,9 @@ int pps_field_copy_create(pps_swarm* s, int32_t field, pps_field_copy** out) {
 int pps_field_copy_read(pps_field_copy* c, float* out) {
   if (!c || !out) return set_error(PPS_EINVAL, "NULL argument");
   PPS_CUDA(cudaSetDevice(c->device));
-  PPS_CUDA(cudaStreamWaitEvent(c->stream, c->ready, 0));
+  PPS_CUDA(cudaStreamWaitEvent(c->ps.stream, c->ps.ev0, 0));
   const size_t w = sizeof(float) * (size_t)c->n;
-  return copy_rows_to_host(c->device, c->stream, reinterpret_cast<char*>(out), reinterpret_cast<const char*>(c->dev),
+  return copy_rows_to_host(c->device, c->ps.stream, reinterpret_cast<char*>(out), reinterpret_cast<const char*>(c->dev),
                            w, w, (size_t)c->rows);
 }
 
@@ -796,14 +808,10 @@ int pps_field_copy_destroy(pps_field_copy* c) {
   if (!c) return PPS_OK;
   cudaSetDevice(c->device);
   if (c->dev) {
-    if (c->stream) cudaStreamWaitEvent(c->stream, c->ready, 0);
-    cudaFreeAsync(c->dev, c->stream);
+    cudaStreamWaitEvent(c->ps.stream, c->ps.ev0, 0);
+    cudaFreeAsync(c->dev, c->ps.stream);
   }
-  if (c->stream) {
-    cudaStreamSynchronize(c->stream);
-    cudaStreamDestroy(c->stream);
-  }
-  if (c->ready) cudaEventDestroy(c->ready);
+  pool_stream_put(c->device, &c->ps);
   delete c;
   return PPS_OK;
 }
@@ -817,14 +825,17 @@ int pps_eval_objective(const pps_problem* prob, int64_t npoints, const float* x,
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return set_error(PPS_ENODEV, "no CUDA device");
   const int D = prob->dim;
   float* dx = nullptr;
-  cudaStream_t st = nullptr;
-  PPS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  int dev = 0;
+  PPS_CUDA(cudaGetDevice(&dev));
+  PoolStream ps;
+  PPS_CUDA(pool_stream_get(dev, &ps));
+  cudaStream_t st = ps.stream;
   // device layout x[d * stride + i]; the stride is padded to 64 points
   const int64_t stride = (int64_t)align_up((size_t)npoints, 64);
   const size_t bx = sizeof(float) * (size_t)D * (size_t)stride;
-  cudaError_t e = cudaMallocAsync(&dx, bx + sizeof(float) * (size_t)stride, st);
+  cudaError_t e = pool_alloc(dev, reinterpret_cast<void**>(&dx), bx + sizeof(float) * (size_t)stride, st);
   if (e != cudaSuccess) {
-    cudaStreamDestroy(st);
+    pool_stream_put(dev, &ps);
     return cuda_error(e, "cudaMallocAsync");
   }
   float* df = dx + (size_t)D * (size_t)stride;
@@ -833,7 +844,7 @@ int pps_eval_objective(const pps_problem* prob, int64_t npoints, const float* x,
   float* ddata = nullptr;
   rc = PPS_OK;
   if (is_ode(prob->objective) || (is_user(prob->objective) && prob->ndata > 0)) {
-    if ((e = cudaMallocAsync(&ddata, sizeof(float) * (size_t)prob->ndata, st)) != cudaSuccess) rc = cuda_error(e, "cudaMallocAsync");
+    if ((e = pool_alloc(dev, reinterpret_cast<void**>(&ddata), sizeof(float) * (size_t)prob->ndata, st)) != cudaSuccess) rc = cuda_error(e, "cudaMallocAsync");
     if (!rc && (e = cudaMemcpyAsync(ddata, prob->data, sizeof(float) * (size_t)prob->ndata, cudaMemcpyHostToDevice, st)) != cudaSuccess)
       rc = cuda_error(e, "cudaMemcpy");
     od.data = ddata;
@@ -845,8 +856,9 @@ int pps_eval_objective(const pps_problem* prob, int64_t npoints, const float* x,
     const int S = (int)(prob->ndata / 17);
     packed.resize(mlp_a_bytes(S));
     mlp_pack_a(prob->data, S, packed.data());
-    if ((e = cudaMallocAsync(&ddata, sizeof(float) * (size_t)prob->ndata, st)) != cudaSuccess ||
-        (e = cudaMallocAsync(&da, packed.size() + 256, st)) != cudaSuccess)
+    if ((e = pool_alloc(dev, reinterpret_cast<void**>(&ddata), sizeof(float) * (size_t)prob->ndata, st)) !=
+            cudaSuccess ||
+        (e = pool_alloc(dev, reinterpret_cast<void**>(&da), packed.size() + 256, st)) != cudaSuccess)
       rc = cuda_error(e, "cudaMallocAsync");
     if (!rc && ((e = cudaMemcpyAsync(ddata, prob->data, sizeof(float) * (size_t)prob->ndata, cudaMemcpyHostToDevice,
                                      st)) != cudaSuccess ||
@@ -880,7 +892,7 @@ int pps_eval_objective(const pps_problem* prob, int64_t npoints, const float* x,
   if (ddata) cudaFreeAsync(ddata, st);
   if (da) cudaFreeAsync(da, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess && !rc) rc = cuda_error(e, "cudaStreamSynchronize");
-  cudaStreamDestroy(st);
+  pool_stream_put(dev, &ps);
   if (!rc && (status & 2u)) rc = set_error(PPS_ETIMEOUT, "the MLP tensor-core kernel timed out waiting for an MMA");
   return rc;
 }

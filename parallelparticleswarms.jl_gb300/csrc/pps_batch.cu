@@ -793,9 +793,16 @@ struct pps_batch {
   int last_threads = 0, last_ppt = 0, last_spread = 8;
   int last_groups = 0, last_max_cluster = 0;
   bool ran = false;
+  float* io = nullptr;  // device: every swarm's g and result words, then every swarm's inputs
+  size_t io_cap = 0;    // floats
+  std::vector<size_t> out_at;    // per swarm: its outputs' place in io
+  size_t out_floats = 0;
+  std::vector<float> outputs;    // the last run's outputs
 };
 
 namespace {
+
+constexpr int kResultWords = 3;  // cost, index bits, iterations
 
 std::mutex g_tune_mu;
 std::map<std::string, std::tuple<int, int, int>> g_tune_cache;  // shape -> (threads, ppt, spread)
@@ -819,23 +826,55 @@ int prepare(pps_batch* b) {
     PPS_CUDA(cudaMalloc(&b->dorder, sizeof(int) * ns));
     b->dcap = ns;
   }
+  // every swarm's inputs (lb | ub | u0 | data) in one block written by one
+  // copy, and its outputs (g, then the result words) in one read by one copy
+  // after the run: a copy per swarm and array took 4 ms of a run of 256 swarms,
+  // reading the results one by one 5 ms
+  size_t nin = 0, nout = 0;
+  for (size_t k = 0; k < ns; ++k) {
+    nin += b->host[k].size();
+    nout += (size_t)b->descs[k].dim + kResultWords;
+  }
+  if (b->io_cap < nin + nout) {
+    if (b->io) cudaFree(b->io);
+    b->io = nullptr;
+    b->io_cap = 0;
+    PPS_CUDA(cudaMalloc(&b->io, sizeof(float) * (nin + nout)));
+    b->io_cap = nin + nout;
+  }
+  std::vector<float> staged;
+  staged.reserve(nin);
+  b->out_at.resize(ns);
+  b->out_floats = nout;
   char* base = static_cast<char*>(b->arena);
+  size_t out = 0;
   for (size_t k = 0; k < ns; ++k) {
     BatchSwarm& d = b->descs[k];
     const int D = d.dim;
     batch_carve(d, base + b->offsets[k]);
     d.mail = nullptr;
     d.done = nullptr;
-    const std::vector<float>& h = b->host[k];
-    PPS_CUDA(cudaMemcpyAsync(const_cast<float*>(d.lb), h.data(), sizeof(float) * D, cudaMemcpyHostToDevice, b->stream));
-    PPS_CUDA(cudaMemcpyAsync(const_cast<float*>(d.ub), h.data() + D, sizeof(float) * D, cudaMemcpyHostToDevice, b->stream));
-    PPS_CUDA(cudaMemcpyAsync(const_cast<float*>(d.u0), h.data() + 2 * D, sizeof(float) * D, cudaMemcpyHostToDevice,
-                             b->stream));
-    if (d.ndata)
-      PPS_CUDA(cudaMemcpyAsync(const_cast<float*>(d.data), h.data() + 3 * D, sizeof(float) * (size_t)d.ndata,
-                               cudaMemcpyHostToDevice, b->stream));
+    d.g = b->io + out;
+    d.result = d.g + D;
+    b->out_at[k] = out;
+    out += (size_t)D + kResultWords;
+    const float* in = b->io + nout + staged.size();
+    d.lb = in;
+    d.ub = in + D;
+    d.u0 = in + 2 * D;
+    if (d.ndata) d.data = in + 3 * D;
+    staged.insert(staged.end(), b->host[k].begin(), b->host[k].end());
   }
+  PPS_CUDA(cudaMemcpyAsync(b->io + nout, staged.data(), sizeof(float) * nin, cudaMemcpyHostToDevice, b->stream));
   PPS_CUDA(cudaMemcpyAsync(b->ddescs, b->descs.data(), sizeof(BatchSwarm) * ns, cudaMemcpyHostToDevice, b->stream));
+  return PPS_OK;
+}
+
+// the run's outputs to the host, behind it on b->stream
+int read_outputs(pps_batch* b) {
+  b->outputs.resize(b->out_floats);
+  PPS_CUDA(cudaMemcpyAsync(b->outputs.data(), b->io, sizeof(float) * b->out_floats, cudaMemcpyDeviceToHost, b->stream));
+  PPS_CUDA(cudaStreamSynchronize(b->stream));
   return PPS_OK;
 }
 
@@ -951,6 +990,7 @@ int pps_batch_destroy(pps_batch* b) {
   if (b->arena) cudaFree(b->arena);
   if (b->ddescs) cudaFree(b->ddescs);
   if (b->dorder) cudaFree(b->dorder);
+  if (b->io) cudaFree(b->io);
   ode_teams_destroy(b->teams);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
@@ -995,7 +1035,7 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
     if (taken) {
       PPS_CUDA(cudaEventRecord(b->ev1, b->stream));
       PPS_CUDA(cudaMemcpyAsync(&timed_out, word, sizeof(timed_out), cudaMemcpyDeviceToHost, b->stream));
-      PPS_CUDA(cudaStreamSynchronize(b->stream));
+      if ((rc = read_outputs(b))) return rc;
       if (device_ms) PPS_CUDA(cudaEventElapsedTime(device_ms, b->ev0, b->ev1));
       if (timed_out) return set_error(PPS_ETIMEOUT, "the batch timed out waiting for a fit's iteration");
       b->last_threads = 128;
@@ -1053,7 +1093,7 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
     }
   }
   if ((rc = run_groups(b, threads, ppt, spread, &b->last_groups, &b->last_max_cluster))) return rc;
-  PPS_CUDA(cudaEventSynchronize(b->ev1));
+  if ((rc = read_outputs(b))) return rc;
   if (device_ms) PPS_CUDA(cudaEventElapsedTime(device_ms, b->ev0, b->ev1));
   b->last_threads = threads;
   b->last_ppt = ppt;
@@ -1091,10 +1131,9 @@ int pps_batch_result(pps_batch* b, int32_t slot, float* u, float* cost, int64_t*
   if (slot < 0 || slot >= (int32_t)b->descs.size()) return set_error(PPS_EINVAL, "slot %d out of range", slot);
   if (!b->ran) return set_error(PPS_EINVAL, "batch has not run");
   const BatchSwarm& d = b->descs[slot];
-  float res[3];
-  PPS_CUDA(cudaMemcpyAsync(res, d.result, sizeof(res), cudaMemcpyDeviceToHost, b->stream));
-  if (u) PPS_CUDA(cudaMemcpyAsync(u, d.g, sizeof(float) * d.dim, cudaMemcpyDeviceToHost, b->stream));
-  PPS_CUDA(cudaStreamSynchronize(b->stream));
+  const float* o = b->outputs.data() + b->out_at[slot];
+  const float* res = o + d.dim;
+  if (u) memcpy(u, o, sizeof(float) * d.dim);
   if (cost) *cost = res[0];
   if (idx) {
     uint32_t bits;

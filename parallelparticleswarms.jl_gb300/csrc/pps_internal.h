@@ -10,6 +10,7 @@
 
 #include "../../include/pps.h"
 #include "pps_device.cuh"
+#include "pps_pool.h"
 #include "pps_state.cuh"
 
 namespace pps {
@@ -29,6 +30,7 @@ struct pps_swarm {
   int device = 0;
   cudaStream_t stream = nullptr;
   void* block = nullptr;  // the single device allocation
+  bool pooled = false;    // block came from pool_alloc (freed in the stream's order)
   size_t bytes = 0;
   pps::SwarmDev dv{};
   pps::ObjParams op{};
