@@ -13,7 +13,6 @@
 // (src/ode_pso.jl:18-19), which compares lexicographically; this build
 // clamps each parameter (max.(x, lb), min.(x, ub)) as the other kernels do.
 #include <cmath>
-
 #include <mutex>
 
 #include "pps_internal.h"
@@ -30,23 +29,28 @@ constexpr int kOdeThreads = 128;
 constexpr int kOdeStepMinBlocks = 4;
 constexpr int kOdeMaxDim = 4;
 
-// dynamic shared memory of a launch: the observations (2 floats per save),
-// then the fixed-step Tsit5 saves' weight table (8 floats per save)
+// dynamic shared memory of a launch: the fixed-step Tsit5 saves' weight table
+// (8 floats per save, read as two 128-bit words), then the observations (2
+// floats per save)
 inline size_t ode_dyn_smem(const OdeCfg& c) {
   return sizeof(float) * (size_t)c.nsaves * (c.method == kOdeTsit5 ? 10 : 2);
 }
 
-// the block's dynamic shared memory: the observations at 0, the fixed-step
-// Tsit5 save table behind them.  Kernels index it directly so the compiler
-// keeps its loads in the shared address space.
-extern __shared__ float ode_smem[];
+// the block's dynamic shared memory.  Kernels index it directly so the
+// compiler keeps its loads in the shared address space.
+extern __shared__ __align__(16) float ode_smem[];
+template <int METHOD>
+__device__ __forceinline__ const float* ode_observations(const OdeCfg& c) {
+  return ode_smem + (METHOD == kOdeTsit5 ? 8 * c.nsaves : 0);
+}
 
 // copies the observations to shared memory and builds the save table
 // (fixed-step Tsit5 only); every thread calls it, and it ends in a barrier
 template <int METHOD>
 __device__ __forceinline__ void ode_smem_fill(const OdeCfg& c, const float* __restrict__ data_g) {
-  for (int k = threadIdx.x; k < 2 * c.nsaves; k += blockDim.x) ode_smem[k] = data_g[k];
-  if constexpr (METHOD == kOdeTsit5) tsit5_table_build(c, ode_smem + 2 * c.nsaves);
+  float* data = const_cast<float*>(ode_observations<METHOD>(c));
+  for (int k = threadIdx.x; k < 2 * c.nsaves; k += blockDim.x) data[k] = data_g[k];
+  if constexpr (METHOD == kOdeTsit5) tsit5_table_build(c, ode_smem, (int)threadIdx.x, (int)blockDim.x);
   __syncthreads();
 }
 
@@ -71,8 +75,8 @@ __global__ void __launch_bounds__(kOdeThreads) k_init_ode(SwarmDev s, ObjParams 
                                                           const float* __restrict__ data_g, uint64_t seed,
                                                           int sampler, const float* __restrict__ u0) {
   ode_smem_fill<METHOD>(cfg, data_g);
-  const float* data = ode_smem;
-  const float* tab = ode_smem + 2 * cfg.nsaves;
+  const float* data = ode_observations<METHOD>(cfg);
+  const float* tab = ode_smem;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
   const int D = s.dim;
@@ -112,6 +116,223 @@ __global__ void __launch_bounds__(kOdeThreads) k_init_ode(SwarmDev s, ObjParams 
   if (publish_block_min(key, s.st)) finish_iteration(s, false, 0u, s.st->w);
 }
 
+// The step of a fixed-step Tsit5 fit as a pipeline of warps over 32 particles.
+// A solve is a chain of steps (6 right-hand sides, about 200 cycles each) and,
+// off that chain, the saves' dense output -- three quarters of the
+// instructions at ten saves a step, which one thread per particle ran in
+// between.  Warp 0 moves the particles and takes the steps, a chunk of `K` ahead;
+// warps 2-7 take a step each and evaluate its saves from the stages warp 0
+// left in shared memory, a lane a particle; warp 1 sums the squared errors in save
+// order, the order of tsit5_loss_tab, whose operations these are: equal bits.
+// One barrier a chunk; two buffers each between the stages.  While warp 0 takes
+// the first chunk the others build the save table.
+constexpr int kPipeWarps = 8, kPipeEval = kPipeWarps - 2;
+constexpr int kPipeMaxSaves = 96;    // saves of a chunk
+constexpr int kPipeMaxSteps = 2048;  // steps of a solve
+
+inline __host__ __device__ size_t pipe_smem(int nsaves, int nsteps, int K) {
+  return sizeof(float) * (8 * (size_t)nsaves + 2 * (size_t)nsaves + 2 * (size_t)K * 16 * 32 + 2 * kPipeMaxSaves * 32) +
+         sizeof(int) * ((size_t)nsteps + 2);
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(kPipeWarps * 32) k_step_tsit5_pipe(SwarmDev s, OdeCfg cfg,
+                                                                    const float* __restrict__ data_g, uint64_t seed,
+                                                                    float c1, float c2, int from_position, int K) {
+  IterState* st = s.st;
+  const uint32_t t = st->t;
+  const float w = st->w;
+  const int D = s.dim, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nsaves = cfg.nsaves, nsteps = cfg.nsteps;
+  float* tab = ode_smem;
+  float* data = tab + 8 * nsaves;
+  float* stages = data + 2 * nsaves;                       // [2][K][16][32]
+  float* errors = stages + 2 * K * 16 * 32;                // [2][kPipeMaxSaves][32]
+  int* start = reinterpret_cast<int*>(errors + 2 * kPipeMaxSaves * 32);  // first save of each step
+  const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+  const bool valid = i < s.n;
+  const int64_t il = valid ? i : s.n - 1;  // lanes past the last particle follow it and write nothing
+
+  float p[kOdeMaxDim] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float l = 0.0f, u0 = cfg.u0a, u1 = cfg.u0b, ka[7], kb[7];
+  auto chunk = [&](int c) {  // warp 0: the steps of chunk c
+    float* out = stages + (c & 1) * K * 16 * 32 + lane;
+    for (int k = 0; k < K; ++k) {
+      float n0, n1;
+      tsit5_step<MODEL>(p, l, cfg.dt, u0, u1, ka, kb, n0, n1);
+      out[0] = u0;
+      out[32] = u1;
+#pragma unroll
+      for (int q = 0; q < 7; ++q) {
+        out[(2 + q) * 32] = ka[q];
+        out[(9 + q) * 32] = kb[q];
+      }
+      out += 16 * 32;
+      u0 = n0;
+      u1 = n1;
+      ka[0] = ka[6];
+      kb[0] = kb[6];
+    }
+  };
+  if (warp == 0) {
+    const Rand4 r0 = philox4x32_10((uint32_t)il, 0u, t, kTagStep, (uint32_t)seed, (uint32_t)(seed >> 32));
+    const Rand4 r1 = philox4x32_10((uint32_t)il, 1u, t, kTagStep, (uint32_t)seed, (uint32_t)(seed >> 32));
+    const float ra[4] = {u01(r0.a), u01(r0.c), u01(r1.a), u01(r1.c)};  // r1 draws of dims 0..3
+    const float rb[4] = {u01(r0.b), u01(r0.d), u01(r1.b), u01(r1.d)};  // r2 draws
+    const bool pending = s.flag[il] != 0;
+#pragma unroll
+    for (int d = 0; d < kOdeMaxDim; ++d) {
+      if (d < D) {
+        const int64_t o = (int64_t)d * s.npad + il;
+        const float xd = s.X[o];
+        const float pd = pending ? xd : s.P[o];
+        const float v = velocity(xd, s.V[o], pd, s.g[d], w, c1, c2, ra[d], rb[d]);
+        p[d] = clamp_lb_ub(__fadd_rn(xd, v), s.lb[d], s.ub[d]);
+        __syncwarp();  // lanes that follow the last particle have read it
+        if (valid) {
+          if (pending) s.P[o] = pd;
+          s.X[o] = p[d];
+          s.V[o] = v;
+        }
+      }
+    }
+    l = ode_l(p, cfg);
+    ode_rhs<MODEL>(p, l, u0, u1, ka[0], kb[0]);
+    chunk(0);
+  } else {
+    const int k0 = threadIdx.x - 32, kn = (kPipeWarps - 1) * 32;
+    for (int k = k0; k < 2 * nsaves; k += kn) data[k] = data_g[k];
+    tsit5_table_build(cfg, tab, k0, kn);
+    asm volatile("bar.sync 1, %0;" ::"n"((kPipeWarps - 1) * 32) : "memory");
+    // start[n]: the first save whose step is n or later
+    for (int m = 1 + k0; m < nsaves; m += kn) {
+      const int n = __float_as_int(tab[8 * m]);
+      for (int q = m == 1 ? 0 : __float_as_int(tab[8 * (m - 1)]) + 1; q <= n; ++q) start[q] = m;
+      if (m == nsaves - 1)
+        for (int q = n + 1; q <= nsteps + 1; ++q) start[q] = nsaves;
+    }
+  }
+  __syncthreads();
+  // steps up to the last save's; saves past the last step are never reached
+  int steps = 0;
+  if (nsaves > 1) {
+    const int last = __float_as_int(tab[8 * (nsaves - 1)]);
+    steps = last + 1 < nsteps ? last + 1 : nsteps;
+  }
+  const int chunks = (steps + K - 1) / K;
+  float acc = 0.0f;
+  if (warp == 1) {
+    const float e0 = __fsub_rn(data[0], cfg.u0a), e1 = __fsub_rn(data[1], cfg.u0b);
+    acc = __fadd_rn(__fmul_rn(e0, e0), __fmul_rn(e1, e1));
+  }
+  for (int c = 1; c <= chunks + 1; ++c) {
+    if (warp == 0) {
+      if (c < chunks) chunk(c);
+    } else if (warp == 1) {
+      if (c >= 2) {
+        const int first = (c - 2) * K, end = first + K < steps ? first + K : steps;
+        const float* e = errors + (c & 1) * kPipeMaxSaves * 32 + lane;
+        const int count = start[end] - start[first];
+#pragma unroll 8
+        for (int m = 0; m < count; ++m) acc = __fadd_rn(acc, e[m * 32]);
+      }
+    } else if (c <= chunks) {
+      const int first = (c - 1) * K;
+      for (int k = warp - 2; k < K && first + k < steps; k += kPipeEval) {
+        const float* in = stages + (((c - 1) & 1) * K + k) * 16 * 32 + lane;
+        float a[7], b[7];
+        const float y0 = in[0], y1 = in[32];
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+          a[q] = in[(2 + q) * 32];
+          b[q] = in[(9 + q) * 32];
+        }
+        const int m0 = start[first + k], m1 = start[first + k + 1];
+        float* e = errors + ((c - 1) & 1) * kPipeMaxSaves * 32 + (m0 - start[first]) * 32 + lane;
+#pragma unroll 2
+        for (int m = m0; m < m1; ++m) {
+          const float4 ra = reinterpret_cast<const float4*>(tab)[2 * m];
+          const float4 rb = reinterpret_cast<const float4*>(tab)[2 * m + 1];
+          const float wt[7] = {ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+          const float x0 = __fsub_rn(data[2 * m], tsit5_dense_w(y0, cfg.dt, wt, a));
+          const float x1 = __fsub_rn(data[2 * m + 1], tsit5_dense_w(y1, cfg.dt, wt, b));
+          *e = __fadd_rn(__fmul_rn(x0, x0), __fmul_rn(x1, x1));
+          e += 32;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  unsigned long long key = ~0ull;
+  if (warp == 1 && valid) {
+    float pc = s.pcost[i];
+    const bool improved = acc < pc;
+    pc = improved ? acc : pc;
+    s.pcost[i] = pc;
+    s.cost[i] = acc;
+    s.flag[i] = improved ? 1 : 0;
+    key = argmin_key(pc, (uint32_t)i);
+  }
+  if (publish_block_min(key, st)) finish_iteration(s, from_position != 0, t + 1u, __fmul_rn(w, st->wdamp));
+}
+
+// The step of an adaptive Tsit5 fit with L lanes per particle: all take every
+// step, each evaluates every L-th save (tsit5a_loss), so a swarm too small for one
+// particle per thread to fill the schedulers gets L times the warps.
+template <int MODEL, int L>
+__global__ void __launch_bounds__(kOdeThreads) k_step_tsit5a_lanes(SwarmDev s, OdeCfg cfg,
+                                                                const float* __restrict__ data_g, uint64_t seed,
+                                                                float c1, float c2, int from_position) {
+  IterState* st = s.st;
+  const uint32_t t = st->t;
+  const float w = st->w;
+  const int D = s.dim;
+  ode_smem_fill<kOdeTsit5Adaptive>(cfg, data_g);
+  const float* data = ode_observations<kOdeTsit5Adaptive>(cfg);
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const bool lead = (threadIdx.x & (L - 1)) == 0, valid = i < s.n;
+  const int64_t il = valid ? i : s.n - 1;  // lanes past the last particle follow it and write nothing
+  const Rand4 r0 = philox4x32_10((uint32_t)il, 0u, t, kTagStep, (uint32_t)seed, (uint32_t)(seed >> 32));
+  const Rand4 r1 = philox4x32_10((uint32_t)il, 1u, t, kTagStep, (uint32_t)seed, (uint32_t)(seed >> 32));
+  const float ra[4] = {u01(r0.a), u01(r0.c), u01(r1.a), u01(r1.c)};  // r1 draws of dims 0..3
+  const float rb[4] = {u01(r0.b), u01(r0.d), u01(r1.b), u01(r1.d)};  // r2 draws
+  const bool pending = s.flag[il] != 0;
+  float x[kOdeMaxDim], v[kOdeMaxDim], p[kOdeMaxDim];
+#pragma unroll
+  for (int d = 0; d < kOdeMaxDim; ++d) {
+    x[d] = v[d] = p[d] = 0.0f;
+    if (d < D) {
+      const int64_t o = (int64_t)d * s.npad + il;
+      const float xd = s.X[o];
+      p[d] = pending ? xd : s.P[o];
+      v[d] = velocity(xd, s.V[o], p[d], s.g[d], w, c1, c2, ra[d], rb[d]);
+      x[d] = clamp_lb_ub(__fadd_rn(xd, v[d]), s.lb[d], s.ub[d]);
+    }
+  }
+  const float pc0 = s.pcost[il];
+  const float c = tsit5a_loss<MODEL, L>(x, cfg, data);
+  __syncwarp();  // every lane has read the particle
+  unsigned long long key = ~0ull;
+  if (valid && lead) {
+#pragma unroll
+    for (int d = 0; d < kOdeMaxDim; ++d) {
+      if (d < D) {
+        const int64_t o = (int64_t)d * s.npad + i;
+        if (pending) s.P[o] = p[d];
+        s.X[o] = x[d];
+        s.V[o] = v[d];
+      }
+    }
+    const bool improved = c < pc0;
+    const float pc = improved ? c : pc0;
+    s.pcost[i] = pc;
+    s.cost[i] = c;
+    s.flag[i] = improved ? 1 : 0;
+    key = argmin_key(pc, (uint32_t)i);
+  }
+  if (publish_block_min(key, st)) finish_iteration(s, from_position != 0, t + 1u, __fmul_rn(w, st->wdamp));
+}
+
 template <int MODEL, int METHOD, int PPT>
 __global__ void __launch_bounds__(kOdeThreads, kOdeStepMinBlocks) k_sync_step_ode(SwarmDev s, ObjParams op, OdeCfg cfg,
                                                                const float* __restrict__ data_g, uint64_t seed,
@@ -128,8 +349,8 @@ __global__ void __launch_bounds__(kOdeThreads, kOdeStepMinBlocks) k_sync_step_od
     sub[threadIdx.x] = s.ub[threadIdx.x];
   }
   ode_smem_fill<METHOD>(cfg, data_g);
-  const float* data = ode_smem;
-  const float* tab = ode_smem + 2 * cfg.nsaves;
+  const float* data = ode_observations<METHOD>(cfg);
+  const float* tab = ode_smem;
   const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
   // this thread's particles: i0 (and i0 + blockDim.x) of the block's tile
   const int64_t i0 = (int64_t)blockIdx.x * blockDim.x * PPT + threadIdx.x;
@@ -260,6 +481,8 @@ __global__ void k_eval_ode(ObjParams op, OdeCfg cfg, const float* __restrict__ d
 // per device to the largest observations + save table (init precedes every
 // captured run of a swarm, so captured launches need no attribute call); the
 // other methods stay within the default 48 KB (2 floats per save).
+constexpr int kPipeSmemMax = 200 << 10;
+
 static int ode_set_smem_limit() {
   static std::mutex mu;
   static bool done[64] = {};
@@ -272,6 +495,7 @@ static int ode_set_smem_limit() {
 #define PPS_ODE_SMEM(M)                                                                                         \
   PPS_CUDA(cudaFuncSetAttribute(k_init_ode<M, kOdeTsit5>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));      \
   PPS_CUDA(cudaFuncSetAttribute(k_sync_step_ode<M, kOdeTsit5, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
+  PPS_CUDA(cudaFuncSetAttribute(k_step_tsit5_pipe<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPipeSmemMax));  \
   PPS_CUDA(cudaFuncSetAttribute(k_eval_ode<M, kOdeTsit5>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))
   PPS_ODE_SMEM(kOdeLV);
   PPS_ODE_SMEM(kOdeFHN);
@@ -296,13 +520,75 @@ int launch_init_ode(pps_swarm* s, int sampler, const float* u0_dev) {
   return PPS_OK;
 }
 
+// Lanes per particle of an adaptive fit: eight up to the size at which the
+// extra steps cost what the spread saves gain (LV, us an iteration, 1 / 4 / 8
+// lanes: 500 particles 110 / 95 / 68, 10000 130 / 115 / 94, 20000 140 / 126 / 121,
+// 40000 146 / 177 / 179; FHN 10000 75 / 66 / 42, 40000 111 / 125 / 100).
+constexpr int64_t kAdaptiveLanesMaxN = 24000;
+constexpr int kAdaptiveLanes = 8;
+
+// Steps per chunk of the pipelined fixed-step form, 0 where it does not apply:
+// a swarm that fills the GPU with one particle per thread (us an iteration of
+// 30 steps and 301 saves, one thread / pipeline: 500 particles 28.6 / 12.7,
+// 10000 29.3 / 16.8, 20000 31.3 / 25.6, 40000 35.7 / 39.7), fewer than two
+// saves a step (no dense output to take off the chain), more steps or saves a
+// chunk than it holds.  The save table's steps are found as the kernel finds
+// them.
+constexpr int64_t kPipeMaxN = 28000;
+
+static int pipe_chunk(const OdeCfg& c, int64_t particles) {
+  if (c.method != kOdeTsit5 || particles > kPipeMaxN || c.nsteps > kPipeMaxSteps ||
+      c.nsaves < 2 * (int64_t)c.nsteps)
+    return 0;
+  for (int K : {6, 3, 1}) {
+    if (pipe_smem(c.nsaves, c.nsteps, K) > (size_t)kPipeSmemMax) continue;
+    int most = 0, count = 0, at = 0, n = 0;
+    for (int m = 1; m < c.nsaves; ++m) {
+      const float tm = (float)m * c.save_dt;
+      while (n < c.nsteps && tm > (float)(n + 1) * c.dt) ++n;
+      if (n / K != at) {
+        at = n / K;
+        count = 0;
+      }
+      if (++count > most) most = count;
+    }
+    if (most <= kPipeMaxSaves) return K;
+  }
+  return 0;
+}
+
 int launch_sync_step_ode(pps_swarm* s, float c1, float c2) {
   const OdeCfg c = cfg_of(s);
+  const int from_pos = (s->flags & PPS_FLAG_GBEST_FROM_POSITION) ? 1 : 0;
+  const bool lv = s->objective == kLvFit;
+  if (const int K = pipe_chunk(c, s->dv.n)) {
+    const unsigned blocks = (unsigned)((s->dv.n + 31) / 32);
+    const size_t smem = pipe_smem(c.nsaves, c.nsteps, K);
+    if (lv)
+      k_step_tsit5_pipe<kOdeLV><<<blocks, kPipeWarps * 32, smem, s->stream>>>(s->dv, c, s->od.data, s->seed, c1, c2,
+                                                                            from_pos, K);
+    else
+      k_step_tsit5_pipe<kOdeFHN><<<blocks, kPipeWarps * 32, smem, s->stream>>>(s->dv, c, s->od.data, s->seed, c1, c2,
+                                                                             from_pos, K);
+    PPS_CUDA(cudaGetLastError());
+    return PPS_OK;
+  }
+  if (c.method == kOdeTsit5Adaptive && s->dv.n <= kAdaptiveLanesMaxN) {
+    constexpr int L = kAdaptiveLanes;
+    const unsigned blocks = (unsigned)((s->dv.n * L + kOdeThreads - 1) / kOdeThreads);
+    if (lv)
+      k_step_tsit5a_lanes<kOdeLV, L><<<blocks, kOdeThreads, ode_dyn_smem(c), s->stream>>>(s->dv, c, s->od.data,
+                                                                                         s->seed, c1, c2, from_pos);
+    else
+      k_step_tsit5a_lanes<kOdeFHN, L><<<blocks, kOdeThreads, ode_dyn_smem(c), s->stream>>>(s->dv, c, s->od.data,
+                                                                                          s->seed, c1, c2, from_pos);
+    PPS_CUDA(cudaGetLastError());
+    return PPS_OK;
+  }
   const bool served = !s->owns_memory;  // state carved from a server's arena
   const int ppt = (c.method == kOdeRk4 && (s->dv.npad >= kOdePackedMinParticles || served)) ? 2 : 1;
   const int64_t tile = (int64_t)kOdeThreads * ppt;
   const unsigned blocks = (unsigned)((s->dv.npad + tile - 1) / tile);
-  const int from_pos = (s->flags & PPS_FLAG_GBEST_FROM_POSITION) ? 1 : 0;
   const size_t dsm = ode_dyn_smem(c);
   // the last argument, 1.0f, is the packed losses' run-time one
 #define L_STEP_ODE(M, I)                                                                                   \
@@ -325,8 +611,8 @@ template <int MODEL, int METHOD>
 __global__ void k_eval_ode(ObjParams op, OdeCfg cfg, const float* __restrict__ data_g, const float* __restrict__ x,
                            int64_t npts, int64_t stride, float* __restrict__ f) {
   ode_smem_fill<METHOD>(cfg, data_g);
-  const float* data = ode_smem;
-  const float* tab = ode_smem + 2 * cfg.nsaves;
+  const float* data = ode_observations<METHOD>(cfg);
+  const float* tab = ode_smem;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= npts) return;
   float p[kOdeMaxDim] = {0.0f, 0.0f, 0.0f, 0.0f};

@@ -285,13 +285,13 @@ __device__ __forceinline__ float tsit5_dense(float u, float dt, float th, const 
 // t_m = m save_dt, at theta = (t_m - t_n) / dt, so its continuous-extension
 // weights b_i(theta) are the same for every particle.  Row m (m >= 1) of the
 // table: n(m) (as int bits), then b_1..b_7(theta); saves past the last step
-// get n(m) = nsteps (never reached, as in the step loop).  Built by all threads
-// of a block before the particles' integrations (8 nsaves floats of shared
+// get n(m) = nsteps (never reached, as in the step loop).  Built by `stride`
+// threads of a block (this one `first` of them) before the particles' integrations (8 nsaves floats of shared
 // memory); each weight is the operation sequence tsit5_dense performs.
-__device__ __forceinline__ void tsit5_table_build(const OdeCfg& c, float* tab) {
+__device__ __forceinline__ void tsit5_table_build(const OdeCfg& c, float* tab, int first, int stride) {
   using namespace ts5;
   const float dt = c.dt;
-  for (int m = 1 + (int)threadIdx.x; m < c.nsaves; m += (int)blockDim.x) {
+  for (int m = 1 + first; m < c.nsaves; m += stride) {
     const float tm = __fmul_rn(__int2float_rn(m), c.save_dt);
     // the smallest n with tm <= (n + 1) dt: an estimate, then corrected
     int n = (int)__fdiv_rn(tm, dt) - 1;
@@ -418,9 +418,13 @@ __device__ __forceinline__ float tsit5_err_sum(const float (&k)[7]) {
 }
 
 // SSE of the adaptive Tsit5 solution at t_m = m save_dt against data; steps
-// (accepted and rejected) in *steps when given
-template <int MODEL>
+// (accepted and rejected) in *steps when given.  With L > 1, L lanes of a warp
+// hold the same particle: all take every step, each evaluates every L-th save,
+// and the squared errors are summed in save order by all.
+template <int MODEL, int L = 1>
 __device__ __forceinline__ float tsit5a_loss(const float* p, const OdeCfg& c, const float* data, int* steps = nullptr) {
+  const int lane = threadIdx.x & (L - 1);
+  const unsigned int group = L == 32 ? 0xffffffffu : ((1u << (L & 31)) - 1u) << (threadIdx.x & 31 & ~(L - 1));
   const float inf = __int_as_float(0x7f800000);
   float u0 = c.u0a, u1 = c.u0b;
   float e0 = __fsub_rn(data[0], u0), e1 = __fsub_rn(data[1], u1);
@@ -454,13 +458,34 @@ __device__ __forceinline__ float tsit5a_loss(const float* p, const OdeCfg& c, co
     const float ra = __fdiv_rn(ea, sa), rb = __fdiv_rn(eb, sb);
     const float err = __fsqrt_rn(__fmul_rn(__fmaf_rn(ra, ra, __fmul_rn(rb, rb)), 0.5f));
     if (err <= 1.0f) {
-      while (m < c.nsaves && tm <= tn1) {  // the saves inside (t, t + hh]
-        const float th = __fdiv_rn(__fsub_rn(tm, t), hh);
-        e0 = __fsub_rn(data[2 * m], tsit5_dense(u0, hh, th, ka));
-        e1 = __fsub_rn(data[2 * m + 1], tsit5_dense(u1, hh, th, kb));
-        acc = __fadd_rn(acc, __fadd_rn(__fmul_rn(e0, e0), __fmul_rn(e1, e1)));
-        ++m;
-        tm = __fmul_rn(__int2float_rn(m), c.save_dt);
+      if constexpr (L == 1) {
+        while (m < c.nsaves && tm <= tn1) {  // the saves inside (t, t + hh]
+          const float th = __fdiv_rn(__fsub_rn(tm, t), hh);
+          e0 = __fsub_rn(data[2 * m], tsit5_dense(u0, hh, th, ka));
+          e1 = __fsub_rn(data[2 * m + 1], tsit5_dense(u1, hh, th, kb));
+          acc = __fadd_rn(acc, __fadd_rn(__fmul_rn(e0, e0), __fmul_rn(e1, e1)));
+          ++m;
+          tm = __fmul_rn(__int2float_rn(m), c.save_dt);
+        }
+      } else {
+        for (int cnt = L; cnt == L && m < c.nsaves; m += cnt) {
+          const int mm = m + lane;
+          const float tmm = __fmul_rn(__int2float_rn(mm), c.save_dt);
+          const bool in = mm < c.nsaves && tmm <= tn1;
+          float sq = 0.0f;
+          if (in) {
+            const float th = __fdiv_rn(__fsub_rn(tmm, t), hh);
+            const float x0 = __fsub_rn(data[2 * mm], tsit5_dense(u0, hh, th, ka));
+            const float x1 = __fsub_rn(data[2 * mm + 1], tsit5_dense(u1, hh, th, kb));
+            sq = __fadd_rn(__fmul_rn(x0, x0), __fmul_rn(x1, x1));
+          }
+          cnt = __popc(__ballot_sync(group, in) & group);
+#pragma unroll
+          for (int k = 0; k < L; ++k) {
+            const float v = __shfl_sync(group, sq, k, L);
+            if (k < cnt) acc = __fadd_rn(acc, v);
+          }
+        }
       }
       t = tn1;
       u0 = n0;
