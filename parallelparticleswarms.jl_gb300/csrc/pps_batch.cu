@@ -789,6 +789,7 @@ struct pps_batch {
   int* dorder = nullptr;
   size_t dcap = 0;
   OdeTeams* teams = nullptr;  // ODE fits alone: their units' tables
+  BatchResident* resident = nullptr;  // closed-form swarms alone: their waves' tables
   int tuned_threads = 0, tuned_ppt = 0, tuned_spread = 8;
   int last_threads = 0, last_ppt = 0, last_spread = 8;
   int last_groups = 0, last_max_cluster = 0;
@@ -992,6 +993,7 @@ int pps_batch_destroy(pps_batch* b) {
   if (b->dorder) cudaFree(b->dorder);
   if (b->io) cudaFree(b->io);
   ode_teams_destroy(b->teams);
+  batch_resident_destroy(b->resident);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -1024,21 +1026,30 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
   int rc = prepare(b);
   if (rc) return rc;
   const int ns = (int)b->descs.size();
-  bool all_ode = true;
-  for (const auto& d : b->descs) all_ode = all_ode && is_ode(d.objective);
-  if (all_ode) {  // ODE fits alone have a form of their own, with nothing to tune
-    if (!b->teams && !(b->teams = ode_teams_create())) return set_error(PPS_ENOMEM, "host allocation failed");
+  bool all_ode = true, none_ode = true;
+  for (const auto& d : b->descs) (is_ode(d.objective) ? none_ode : all_ode) = false;
+  int pinned = b->tuned_threads, pin_ppt = 0, pin_spread = 0;
+  if (!pinned) pinned_shape(&pinned, &pin_ppt, &pin_spread);
+  if (all_ode || (none_ode && !pinned)) {
+    // fits alone, and closed-form swarms alone whose block shape nobody has
+    // fixed, have forms of their own, with nothing to tune
+    if (all_ode && !b->teams && !(b->teams = ode_teams_create())) return set_error(PPS_ENOMEM, "host allocation failed");
+    if (none_ode && !b->resident && !(b->resident = batch_resident_create()))
+      return set_error(PPS_ENOMEM, "host allocation failed");
     bool taken = false;
     unsigned int *word = nullptr, timed_out = 0;
     PPS_CUDA(cudaEventRecord(b->ev0, b->stream));
-    if ((rc = ode_teams_launch(b->teams, b->stream, b->descs, b->ddescs, b->sm_count, &taken, &word))) return rc;
+    rc = all_ode ? ode_teams_launch(b->teams, b->stream, b->descs, b->ddescs, b->sm_count, &taken, &word)
+                 : batch_resident_launch(b->resident, b->stream, b->descs, b->host, b->ddescs, b->sm_count, &taken,
+                                         &word);
+    if (rc) return rc;
     if (taken) {
       PPS_CUDA(cudaEventRecord(b->ev1, b->stream));
       PPS_CUDA(cudaMemcpyAsync(&timed_out, word, sizeof(timed_out), cudaMemcpyDeviceToHost, b->stream));
       if ((rc = read_outputs(b))) return rc;
       if (device_ms) PPS_CUDA(cudaEventElapsedTime(device_ms, b->ev0, b->ev1));
-      if (timed_out) return set_error(PPS_ETIMEOUT, "the batch timed out waiting for a fit's iteration");
-      b->last_threads = 128;
+      if (timed_out) return set_error(PPS_ETIMEOUT, "the batch timed out waiting for a swarm's iteration");
+      b->last_threads = all_ode ? 128 : 512;
       b->last_ppt = 1;
       b->ran = true;
       return PPS_OK;

@@ -70,6 +70,15 @@ OdeTeams* ode_teams_create();
 void ode_teams_destroy(OdeTeams* t);
 int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSwarm>& descs, const BatchSwarm* ddescs,
                      int sm_count, bool* taken, unsigned int** error_word);
+// a batch of closed-form swarms alone, resident in shared memory wave by wave
+// (pps_batch_resident.cu); host: per swarm lb | ub | ...  *taken, *error_word
+// as for ode_teams_launch (*taken also false where a swarm does not fit the form).
+struct BatchResident;
+BatchResident* batch_resident_create();
+void batch_resident_destroy(BatchResident* t);
+int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vector<BatchSwarm>& descs,
+                          const std::vector<std::vector<float>>& host, const BatchSwarm* ddescs, int sm_count,
+                          bool* taken, unsigned int** error_word);
 // launch one group: descs[dorder[g.offset + k]], k < g.count, on `stream`
 int batch_launch_group(cudaStream_t stream, const BatchSwarm* ddescs, const int* dorder, const LaunchGroup& g,
                        int ppt);

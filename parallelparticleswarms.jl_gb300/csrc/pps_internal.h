@@ -85,7 +85,9 @@ int launch_async(pps_swarm* s, int iters, float c1, float c2, int* lanes_out);
 int launch_eval(const ObjParams& op, const ObjData& od, int objective, const float* x, int64_t npts,
                 int64_t stride, float* f, cudaStream_t stream);
 int async_lanes(int dim, int* slice);
-bool pair_form(const pps_swarm* s, float c1, float c2);  // whether the arithmetic of pps_pair.cuh is exact for a run
+// whether the arithmetic of pps_pair.cuh is exact for a run
+bool pair_form(const pps_swarm* s, float c1, float c2);
+bool pair_form(int objective, const ObjParams& op, int dim, const float* lb, const float* ub, float c1, float c2);
 int sync_grid(pps_swarm* s);
 // the TMA-staged step (pps_sync_bulk.cu): resident blocks per SM where it
 // applies (0 where it does not), resolved outside any stream capture; the
@@ -102,6 +104,9 @@ struct ResidentPlan {
   bool split;
   size_t smem;
 };
+// the split over `blocks` blocks (or fewer, all full) of at most `most` threads
+// and `smem` bytes of dynamic shared memory; false: it does not fit
+bool resident_fit(int objective, int dim, int64_t n, bool cons, int blocks, int most, size_t smem, ResidentPlan* p);
 bool resident_plan(int objective, int dim, int64_t n, int ncons, int sm_count, ResidentPlan* p);
 size_t resident_exchange_bytes(int objective, int dim, int64_t n, int ncons, int sm_count);
 // *taken false: the device could not hold the grid, nothing was launched

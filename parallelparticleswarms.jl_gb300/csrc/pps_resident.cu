@@ -19,12 +19,9 @@ namespace pps {
 template <int OBJ, bool SPLIT, bool CONS>
 __global__ void __launch_bounds__(kResidentMaxThreads, 1)
     k_resident(SwarmDev s, ObjParams op, PhiloxKeys keys, ResidentArgs a) {
-  resident_run<OBJ, SPLIT, CONS>(s, op, keys, a);
+  resident_run<OBJ, SPLIT, CONS>(s, op, keys, a, (int)blockIdx.x);
 }
 
-// polls of one word before a wait gives up: each is at least an L2 round trip
-// (several hundred cycles), so seconds -- no exchange takes milliseconds
-constexpr unsigned int kResidentPollLimit = 1u << 23;
 // a user objective may take its own time, and unevenly: minutes
 constexpr unsigned int kResidentUserPollLimit = 1u << 29;
 constexpr size_t kResidentSmem = 227u << 10;  // a block's shared memory, static part included
@@ -43,16 +40,15 @@ size_t resident_exchange_bytes(int objective, int dim, int64_t n, int ncons, int
   return sizeof(unsigned long long) * 2 * resident_words(p.blocks, dim);
 }
 
-static bool resident_fit(int objective, int dim, int64_t n, bool cons, int blocks, ResidentPlan* p) {
+bool resident_fit(int objective, int dim, int64_t n, bool cons, int blocks, int most, size_t smem, ResidentPlan* p) {
   const int64_t chunk = (n + blocks - 1) / blocks;
   const int np = (dim + 1) / 2;
-  const int most = is_user(objective) ? kResidentUserThreads : kResidentMaxThreads;
   if (chunk > (1 << 20)) return false;
   int groups = (int)(most / chunk);
   if (groups > np) groups = np;
   if (groups > 1) groups = (np + (np + groups - 1) / groups - 1) / ((np + groups - 1) / groups);  // even shares
   bool split = cons || groups > 1;
-  if (!cons && split && resident_smem(dim, (int)chunk, terms_moved(objective)) + kResidentStatic > kResidentSmem) {
+  if (!cons && split && resident_smem(dim, (int)chunk, terms_moved(objective)) > smem) {
     split = false;  // no room for the terms: one thread walks all dims
   }
   split = split || is_user(objective);
@@ -65,7 +61,7 @@ static bool resident_fit(int objective, int dim, int64_t n, bool cons, int block
   const int64_t rounds = (want + most - 1) / most;
   p->threads = (int)(((want + rounds - 1) / rounds + 31) / 32 * 32);
   p->smem = resident_smem(dim, (int)chunk, split && terms_moved(objective));
-  if (p->smem + kResidentStatic > kResidentSmem) return false;
+  if (p->smem > smem) return false;
   return true;
 }
 
@@ -90,8 +86,9 @@ bool resident_plan(int objective, int dim, int64_t n, int ncons, int sm_count, R
   if (is_user(objective)) blocks = (n + 31) / 32;
   if (blocks > sm_count) blocks = sm_count;
   if (blocks > n) blocks = n;
-  return resident_fit(objective, dim, n, ncons > 0, (int)blocks, p) ||
-         resident_fit(objective, dim, n, ncons > 0, sm_count, p);
+  const int most = is_user(objective) ? kResidentUserThreads : kResidentMaxThreads;
+  return resident_fit(objective, dim, n, ncons > 0, (int)blocks, most, kResidentSmem - kResidentStatic, p) ||
+         resident_fit(objective, dim, n, ncons > 0, sm_count, most, kResidentSmem - kResidentStatic, p);
 }
 
 static int launch_one(const void* kernel, pps_swarm* s, const ResidentPlan& p, PhiloxKeys keys, ResidentArgs a,
@@ -137,6 +134,7 @@ int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w,
   *taken = false;
   ResidentArgs a{};
   a.chunk = p.chunk;
+  a.blocks = p.blocks;
   a.groups = p.groups;
   a.iters = iters;
   a.t0 = s->t;
@@ -149,6 +147,7 @@ int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w,
   a.poll_limit = kResidentPollLimit;
   a.one = 1.0f;
   a.xch = s->xch_dev;
+  a.status = &s->dv.st->status;
   const PhiloxKeys keys = philox_round_keys(s->seed);
   int rc;
   if (is_user(s->objective)) {

@@ -37,6 +37,7 @@ namespace pps {
 
 struct ResidentArgs {
   int chunk;          // particles of a block
+  int blocks;         // blocks that share the swarm
   int groups;         // threads that share a particle's pairs
   int iters;
   uint32_t t0;
@@ -46,7 +47,8 @@ struct ResidentArgs {
   uint32_t seq0;      // sequence number before the first exchange
   unsigned int poll_limit;
   float one;          // 1.0f (pps_pair.cuh)
-  unsigned long long* xch;  // exchange of a grid of several blocks: two buffers of resident_words
+  unsigned long long* xch;  // exchange of several blocks: two buffers of resident_words
+  unsigned int* status;     // a wait that gives up sets kStatusResidentTimeout here
 };
 
 // objectives whose terms are computed while moving in the SPLIT form
@@ -54,6 +56,9 @@ template <int OBJ>
 constexpr bool kTermsMoved = OBJ == kRastrigin || OBJ == kAckley;
 
 constexpr int kResidentMaxThreads = 1024;
+// polls of one word before a wait gives up: each is at least an L2 round trip
+// (several hundred cycles), so seconds -- no exchange takes milliseconds
+constexpr unsigned int kResidentPollLimit = 1u << 23;
 constexpr int kResidentUserThreads = 512;  // 128 registers for a user objective
 
 // shared memory of a block: bounds (float4 per pair), g (float2 per pair),
@@ -174,10 +179,14 @@ __device__ __forceinline__ float coord_get(const float2* A, int d, int p, int ch
   return reinterpret_cast<const float*>(A)[ROWS ? d * chunk + p : 2 * ((d >> 1) * chunk + p) + (d & 1)];
 }
 
-// `prm8`: a user objective's 8 parameters in shared memory
+// The run of swarm `s` by the a.blocks blocks that hold it, this one block
+// `rank` of them.  s.flag and s.st may be NULL (a batched swarm): no pending
+// copies, and the global best goes to `result` (cost, index bits, iterations).
+// `prm8`: a user objective's 8 parameters in shared memory.
 template <int OBJ, bool SPLIT, bool CONS>
 __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams& op, const PhiloxKeys& keys,
-                                             const ResidentArgs& a, const float* prm8 = nullptr) {
+                                             const ResidentArgs& a, int rank, float* result = nullptr,
+                                             const float* prm8 = nullptr) {
   static_assert(SPLIT || !(CONS || OBJ == kUserObjective), "constraints and user objectives are summed in a phase of their own");
   constexpr bool ROWS = OBJ == kUserObjective;
   extern __shared__ __align__(16) float rsm[];
@@ -186,7 +195,7 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
   __shared__ int bail;
   const int D = s.dim, np = (D + 1) >> 1, chunk = a.chunk;
   const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
-  const int64_t first = (int64_t)blockIdx.x * chunk;
+  const int64_t first = (int64_t)rank * chunk;
   int cnt = (int)(s.n - first < (int64_t)chunk ? s.n - first : (int64_t)chunk);
   cnt = cnt < 0 ? 0 : cnt;
   constexpr bool TERMS = SPLIT && kTermsMoved<OBJ>;
@@ -208,7 +217,7 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
   }
   for (int p = tid; p < cnt; p += T) {
     pcost[p] = s.pcost[first + p];
-    flag[p] = s.flag[first + p];
+    flag[p] = s.flag ? s.flag[first + p] : 0;
   }
   if (tid == 0) bail = 0;
   for (int p = lane; p < cnt; p += 32) {  // a warp per pair row
@@ -340,7 +349,7 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     if (!none) src = (a.from_position || flag[lp]) ? X : P;
     // ---- agree on the global best
     const uint32_t seq = a.seq0 + 1u + (uint32_t)it;
-    const int nb = (int)gridDim.x;
+    const int nb = a.blocks;
     unsigned long long* kw = a.xch + (size_t)par * resident_words(nb, D);  // keys
     unsigned long long* vw = kw + 2 * (size_t)nb;                          // vectors
     if (nb == 1) {
@@ -348,12 +357,12 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
       for (int d = tid; d < D; d += T) gs[d] = coord_get<ROWS>(src, d, lp, chunk);
     } else {
       if (tid == 0) {
-        post_word(kw + 2 * (size_t)blockIdx.x, resident_word((uint32_t)(mine >> 32), seq));
-        post_word(kw + 2 * (size_t)blockIdx.x + 1, resident_word((uint32_t)mine, seq));
+        post_word(kw + 2 * (size_t)rank, resident_word((uint32_t)(mine >> 32), seq));
+        post_word(kw + 2 * (size_t)rank + 1, resident_word((uint32_t)mine, seq));
       }
       if (!none)
         for (int d = tid; d < D; d += T)
-          post_word(vw + (size_t)blockIdx.x * D + d,
+          post_word(vw + (size_t)rank * D + d,
                     resident_word(__float_as_uint(coord_get<ROWS>(src, d, lp, chunk)), seq));
     }
     if (nb > 1 && warp == 0) {
@@ -374,7 +383,7 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
         win_s = k;
         if (!ok) {
           bail = 1;
-          atomicOr(&s.st->status, kStatusResidentTimeout);
+          atomicOr(a.status, kStatusResidentTimeout);
         }
       }
     }
@@ -407,20 +416,27 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
   }
   for (int p = tid; p < cnt; p += T) {
     s.pcost[first + p] = pcost[p];
-    s.flag[first + p] = 0;
+    if (s.flag) s.flag[first + p] = 0;
   }
-  if (blockIdx.x == 0) {
+  if (rank == 0) {
     for (int d = tid; d < D; d += T) s.g[d] = gs[d];
     if (tid == 0) {
       const uint32_t o = (uint32_t)(win >> 32);
-      s.st->gcost = __uint_as_float((o & 0x80000000u) ? (o ^ 0x80000000u) : ~o);
-      s.st->gidx = (uint32_t)win;
-      s.st->key = ~0ull;
-      s.st->count = 0u;
-      s.st->tile_next = 0u;
-      s.st->t = a.t0 + (uint32_t)a.iters;
-      s.st->w = w;
-      s.st->wdamp = a.wdamp;
+      const float gcost = __uint_as_float((o & 0x80000000u) ? (o ^ 0x80000000u) : ~o);
+      if (result) {
+        result[0] = gcost;
+        result[1] = __uint_as_float((uint32_t)win);
+        result[2] = (float)a.iters;
+      } else {
+        s.st->gcost = gcost;
+        s.st->gidx = (uint32_t)win;
+        s.st->key = ~0ull;
+        s.st->count = 0u;
+        s.st->tile_next = 0u;
+        s.st->t = a.t0 + (uint32_t)a.iters;
+        s.st->w = w;
+        s.st->wdamp = a.wdamp;
+      }
     }
   }
 }

@@ -279,7 +279,7 @@ extern "C" __global__ void __launch_bounds__(pps::kResidentUserThreads, 1)
   __shared__ float sp[8];
   pps::user_params(sp, op);
   __syncthreads();
-  pps::resident_run<pps::kUserObjective, true, true>(s, op, keys, a, sp);
+  pps::resident_run<pps::kUserObjective, true, true>(s, op, keys, a, (int)blockIdx.x, nullptr, sp);
 }
 
 // ParallelPSOKernel(global_update = false) for a user objective: the whole run
