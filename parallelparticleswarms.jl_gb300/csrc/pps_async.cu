@@ -306,19 +306,20 @@ int async_lanes(int dim, int* slice) {
 // whether the shorter arithmetic of the pair forms is exact for this run: the
 // coefficients scale (coef_scales), no bound is a negative zero (clamp_box) and
 // the cosines' arguments stay below cos2pi_box's limit
-bool pair_form(int objective, const ObjParams& op, int dim, const float* lb, const float* ub, float c1, float c2) {
-  if (!coef_scales(c1) || !coef_scales(c2)) return false;
-  const bool cosines = objective == kRastrigin || objective == kAckley;
+bool box_cosines(int objective, const ObjParams& op, int dim, const float* lb, const float* ub) {
+  if (objective != kRastrigin && objective != kAckley) return true;
   const float k = objective == kAckley ? fabsf(op.np > 2 ? op.p[2] : 1.0f) : 1.0f;
   for (int d = 0; d < dim; ++d) {
-    const float lo = lb[d], hi = ub[d];
-    if ((lo == 0.0f && std::signbit(lo)) || (hi == 0.0f && std::signbit(hi))) return false;
-    if (cosines) {
-      const float m = fmaxf(fabsf(lo), fabsf(hi));
-      if (!(m < kCosBoxLimit) || !(m * k < kCosBoxLimit)) return false;
-    }
+    const float m = fmaxf(fabsf(lb[d]), fabsf(ub[d]));
+    if (!(m < kCosBoxLimit) || !(m * k < kCosBoxLimit)) return false;
   }
   return true;
+}
+bool pair_form(int objective, const ObjParams& op, int dim, const float* lb, const float* ub, float c1, float c2) {
+  if (!coef_scales(c1) || !coef_scales(c2)) return false;
+  for (int d = 0; d < dim; ++d)
+    if ((lb[d] == 0.0f && std::signbit(lb[d])) || (ub[d] == 0.0f && std::signbit(ub[d]))) return false;
+  return box_cosines(objective, op, dim, lb, ub);
 }
 bool pair_form(const pps_swarm* s, float c1, float c2) {
   return pair_form(s->objective, s->op, s->dv.dim, s->host_lb, s->host_ub, c1, c2);

@@ -215,7 +215,10 @@ static int launch_local_obj(pps_swarm* s, int kind, const float* x0, const Local
   if constexpr (OBJ >= kBeale) {  // closed forms are defined for dim <= 2
     rc = launch_local_t<OBJ, 2>(s, kind, x0, o, b);
   } else {
-    if (D <= 2) rc = launch_local_t<OBJ, 2>(s, kind, x0, o, b);
+    // the cosines' bounded form needs moderate bounds; others take the widest kernel
+    const bool wide = kind == 0 && !box_cosines(OBJ, s->op, D, s->host_lb, s->host_ub);
+    if (wide) rc = launch_local_lbfgs<OBJ, 64>(s, x0, o, b);
+    else if (D <= 2) rc = launch_local_t<OBJ, 2>(s, kind, x0, o, b);
     else if (D <= 4) rc = launch_local_t<OBJ, 4>(s, kind, x0, o, b);
     else if (D <= 8) rc = launch_local_t<OBJ, 8>(s, kind, x0, o, b);
     else if (D <= 10) rc = kind == 0 ? launch_local_lbfgs<OBJ, 10>(s, x0, o, b)

@@ -87,6 +87,8 @@ int launch_eval(const ObjParams& op, const ObjData& od, int objective, const flo
 int async_lanes(int dim, int* slice);
 // whether the arithmetic of pps_pair.cuh is exact for a run
 bool pair_form(const pps_swarm* s, float c1, float c2);
+// (box_cosines: the part of it about the cosines' arguments inside the bounds)
+bool box_cosines(int objective, const ObjParams& op, int dim, const float* lb, const float* ub);
 bool pair_form(int objective, const ObjParams& op, int dim, const float* lb, const float* ub, float c1, float c2);
 int sync_grid(pps_swarm* s);
 // the TMA-staged step (pps_sync_bulk.cu): resident blocks per SM where it

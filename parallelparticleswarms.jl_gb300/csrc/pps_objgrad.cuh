@@ -15,23 +15,30 @@ namespace pps {
 // arrays of the caller stay in registers.
 #define PPS_FOR_D(d) _Pragma("unroll") for (int d = 0; d < MAXD; ++d) if (d < D)
 
-template <int OBJ, int MAXD>
-__device__ __forceinline__ float obj_value(const ObjParams& op, const float (&x)[MAXD], int D) {
+// f(x); s1 and s2 receive its sums over the dims (Ackley's gradient starts from
+// them).  BOX: see Acc.
+template <int OBJ, int MAXD, bool BOX = false>
+__device__ __forceinline__ float obj_value(const ObjParams& op, const float (&x)[MAXD], int D, float& s1, float& s2) {
 #ifdef PPS_USER_SOURCE
   if constexpr (OBJ == kUserObjective) return pps_objective(pps_point{x, 1}, D, op.p, op.data, op.ndata);
 #endif
-  Acc<OBJ> acc;
+  Acc<OBJ, BOX> acc;
   PPS_FOR_D(d) acc.add(op, d, x[d]);
+  s1 = acc.s1;
+  s2 = acc.s2;
   return finalize<OBJ>(op, acc.s1, acc.s2);
 }
+template <int OBJ, int MAXD, bool BOX = false>
+__device__ __forceinline__ float obj_value(const ObjParams& op, const float (&x)[MAXD], int D) {
+  float s1, s2;
+  return obj_value<OBJ, MAXD, BOX>(op, x, D, s1, s2);
+}
 
-// f(x) and grad f(x) into g[0..D)
+// grad f(x) into g[0..D) of a registered objective, s1 and s2 the sums of
+// obj_value at x
 template <int OBJ, int MAXD>
-__device__ __forceinline__ float obj_grad(const ObjParams& op, const float (&x)[MAXD], float (&g)[MAXD], int D) {
-#if defined(PPS_USER_SOURCE) && defined(PPS_HAS_GRADIENT)
-  if constexpr (OBJ == kUserObjective) return pps_gradient(pps_point{x, 1}, D, op.p, op.data, op.ndata, g);
-#endif
-  const float f = obj_value<OBJ, MAXD>(op, x, D);
+__device__ __forceinline__ void obj_gradient(const ObjParams& op, const float (&x)[MAXD], float (&g)[MAXD], int D,
+                                             float s1, float s2) {
   if constexpr (OBJ == kSphere) {
     PPS_FOR_D(d) g[d] = __fmul_rn(2.0f, x[d]);
   } else if constexpr (OBJ == kRosenbrock) {
@@ -54,11 +61,6 @@ __device__ __forceinline__ float obj_grad(const ObjParams& op, const float (&x)[
   } else if constexpr (OBJ == kAckley) {
     const float a = prm(op, 0, 20.0f), b = prm(op, 1, 0.2f), k = prm(op, 2, 1.0f);
     const float Df = (float)D;
-    float s1 = 0.0f, s2 = 0.0f;
-    PPS_FOR_D(d) {
-      s1 = __fadd_rn(s1, __fmul_rn(x[d], x[d]));
-      s2 = __fadd_rn(s2, cos2pi(__fmul_rn(k, x[d])));
-    }
     const float rms = __fsqrt_rn(__fdiv_rn(s1, Df));
     const float e1 = exp_f(__fmul_rn(-b, rms));
     const float e2 = exp_f(__fdiv_rn(s2, Df));
@@ -97,6 +99,17 @@ __device__ __forceinline__ float obj_grad(const ObjParams& op, const float (&x)[
     g[0] = __fmul_rn(2.0f, __fadd_rn(x[0], 1.0f));
     PPS_FOR_D(d) if (d > 0) g[d] = 0.0f;
   }
+}
+
+// f(x) and grad f(x) into g[0..D)
+template <int OBJ, int MAXD, bool BOX = false>
+__device__ __forceinline__ float obj_grad(const ObjParams& op, const float (&x)[MAXD], float (&g)[MAXD], int D) {
+#if defined(PPS_USER_SOURCE) && defined(PPS_HAS_GRADIENT)
+  if constexpr (OBJ == kUserObjective) return pps_gradient(pps_point{x, 1}, D, op.p, op.data, op.ndata, g);
+#endif
+  float s1, s2;
+  const float f = obj_value<OBJ, MAXD, BOX>(op, x, D, s1, s2);
+  obj_gradient<OBJ, MAXD>(op, x, g, D, s1, s2);
   return f;
 }
 
