@@ -13,12 +13,13 @@
 // wait for each other are all resident.
 //
 // Measured on a GB300, ms a batch of 300 iterations, streaming -> resident: 16
-// swarms of the mix above 8.3 -> 1.6, 32 8.1 -> 1.8, 64 8.4 -> 3.3, 128 13.0 ->
-// 7.2, 256 13.8 -> 12.5, 512 26.4 -> 27.1 (streaming fills the GPU by then); 256
-// with 100 to 2000 iterations 77 -> 55; 500 swarms of 100-600 x 2-20 3.9 -> 3.3;
+// swarms of the mix above 8.3 -> 1.5, 32 8.1 -> 1.6, 64 8.4 -> 2.9, 128 13.0 ->
+// 7.0, 256 13.8 -> 11.7, 512 26.4 -> 27 (streaming fills the GPU by then); 256
+// with 100 to 2000 iterations 77 -> 49; 500 swarms of 100-600 x 2-20 3.9 -> 3.2;
 // 1000 of 50-300 x 2-5 1.6 -> 2.2 (an SM runs several such swarms at once when
 // streaming); 64 of 100-500 x 100-400 15.8 -> 16.8 (few particles a block, a long
-// sum each).
+// sum each).  Blocks of 512 threads with two pairs unrolled; of 1024: 12.5 for
+// the 256 swarms, 55 for the uneven ones.
 #include <algorithm>
 #include <new>
 #include <queue>
@@ -114,13 +115,13 @@ __global__ void __launch_bounds__(kBatchInitThreads) k_batch_init(const BatchSwa
 template <int OBJ>
 __device__ __forceinline__ void run_job(const ResidentJob& j, int rank) {
   if (j.split)
-    resident_run<OBJ, true, false>(j.s, j.op, j.keys, j.a, rank, j.result);
+    resident_run<OBJ, true, false, 2>(j.s, j.op, j.keys, j.a, rank, j.result);
   else
-    resident_run<OBJ, false, false>(j.s, j.op, j.keys, j.a, rank, j.result);
+    resident_run<OBJ, false, false, 2>(j.s, j.op, j.keys, j.a, rank, j.result);
 }
 
 // blocks[b]: the job and the rank in it of block b
-__global__ void __launch_bounds__(kResidentMaxThreads, 1)
+__global__ void __launch_bounds__(kResidentThreads, 1)
     k_batch_resident(const ResidentJob* __restrict__ jobs, const int2* __restrict__ blocks) {
   __shared__ __align__(16) ResidentJob job;
   const int2 at = blocks[blockIdx.x];
@@ -149,7 +150,7 @@ void batch_resident_destroy(BatchResident* t) {
 
 // the blocks' limits with `per` of them on an SM
 constexpr size_t kJobStatic = 6u << 10;  // static shared memory of k_batch_resident, and the driver's 1 kB a block
-static int most_threads(int per) { return kResidentMaxThreads / per; }
+static int most_threads(int per) { return kResidentThreads / per; }
 static size_t most_smem(int per) { return ((size_t)(227u << 10) / per - kJobStatic) / 16 * 16; }
 static bool job_fit(const BatchSwarm& d, int blocks, int per, ResidentPlan* p) {
   return resident_fit(d.objective, d.dim, d.n, false, blocks, most_threads(per), most_smem(per), p);
@@ -161,7 +162,7 @@ int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vect
                           bool* taken, unsigned int** error_word) {
   *taken = false;
   const int ns = (int)descs.size();
-  // blocks per SM: one of 1024 threads, or more and smaller ones while the
+  // blocks per SM: one of 512 threads, or more and smaller ones while the
   // swarms are small (a block of few coordinates waits for its own latencies)
   int64_t coords = 0;
   for (const auto& d : descs) {

@@ -2,12 +2,12 @@
 // for the whole run (pps_resident.cuh), and how they are launched.
 //
 // Measured on a GB300, us an iteration, one launch per iteration -> resident:
-// Rosenbrock 1000 x 3 7.2 -> 1.7, Rastrigin 10000 x 10 9.4 -> 2.3, Ackley
-// 20011 x 30 16.2 -> 4.4, Rosenbrock 65536 x 10 9.4 -> 3.9, sphere 100003 x 20
-// 18.2 -> 5.5, Rastrigin 10000 x 100 36.1 -> 5.5, 250000 x 10 19.6 -> 8.8,
-// 20011 x 128 45.5 -> 14.7 (the pair arithmetic of pps_pair.cuh took the last
-// three large ones from 5.9, 9.6 and 16.4; the small ones wait for the
-// exchange, 2100 cycles of 3700 at 1000 x 3, 3300 of 9100 at 20011 x 30).  The
+// Rosenbrock 1000 x 3 7.2 -> 1.5, Rastrigin 10000 x 10 9.4 -> 2.0, Ackley
+// 20011 x 30 16.2 -> 3.9, Rosenbrock 65536 x 10 9.4 -> 3.6, sphere 100003 x 20
+// 18.2 -> 5.5, Rastrigin 10000 x 100 36.1 -> 4.9, 250000 x 10 19.6 -> 9.0,
+// 20011 x 128 45.5 -> 14.9 (the pair arithmetic of pps_pair.cuh took large ones
+// from 5.9, 9.6 and 16.4; the small ones wait for the exchange, 2100 cycles of
+// 3700 at 1000 x 3, 3300 of 9100 at 20011 x 30).  The
 // line is the shared memory of all SMs (about 2.8 M coordinates of 12 bytes,
 // 2.1 M with the moved terms): beyond it the state has to stream from L2 or
 // memory each iteration, which k_sync_step does.
@@ -16,8 +16,8 @@
 
 namespace pps {
 
-template <int OBJ, bool SPLIT, bool CONS>
-__global__ void __launch_bounds__(kResidentMaxThreads, 1)
+template <int OBJ, bool SPLIT, bool CONS, int T = kResidentThreads>
+__global__ void __launch_bounds__(T, 1)
     k_resident(SwarmDev s, ObjParams op, PhiloxKeys keys, ResidentArgs a) {
   resident_run<OBJ, SPLIT, CONS>(s, op, keys, a, (int)blockIdx.x);
 }
@@ -86,9 +86,14 @@ bool resident_plan(int objective, int dim, int64_t n, int ncons, int sm_count, R
   if (is_user(objective)) blocks = (n + 31) / 32;
   if (blocks > sm_count) blocks = sm_count;
   if (blocks > n) blocks = n;
-  const int most = is_user(objective) ? kResidentUserThreads : kResidentMaxThreads;
-  return resident_fit(objective, dim, n, ncons > 0, (int)blocks, most, kResidentSmem - kResidentStatic, p) ||
-         resident_fit(objective, dim, n, ncons > 0, sm_count, most, kResidentSmem - kResidentStatic, p);
+  for (const int64_t b : {blocks, (int64_t)sm_count}) {
+    // the constrained and the user form have the narrow kernel only
+    const bool wide = !is_user(objective) && ncons == 0 && (n + b - 1) / b > kResidentThreads;
+    if (resident_fit(objective, dim, n, ncons > 0, (int)b, wide ? kResidentMaxThreads : kResidentThreads,
+                     kResidentSmem - kResidentStatic, p))
+      return true;
+  }
+  return false;
 }
 
 static int launch_one(const void* kernel, pps_swarm* s, const ResidentPlan& p, PhiloxKeys keys, ResidentArgs a,
@@ -126,6 +131,9 @@ static int launch_obj(pps_swarm* s, const ResidentPlan& p, const PhiloxKeys& key
   if constexpr (OBJ < kBeale) {
     if (p.split) return launch_one(reinterpret_cast<const void*>(k_resident<OBJ, true, false>), s, p, keys, a, taken);
   }
+  if (p.threads > kResidentThreads)
+    return launch_one(reinterpret_cast<const void*>(k_resident<OBJ, false, false, kResidentMaxThreads>), s, p, keys, a,
+                      taken);
   return launch_one(reinterpret_cast<const void*>(k_resident<OBJ, false, false>), s, p, keys, a, taken);
 }
 

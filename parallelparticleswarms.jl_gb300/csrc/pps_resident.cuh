@@ -55,11 +55,16 @@ struct ResidentArgs {
 template <int OBJ>
 constexpr bool kTermsMoved = OBJ == kRastrigin || OBJ == kAckley;
 
+// Threads of a block: up to 512, with 128 registers each, while a block has at
+// most so many particles, else up to 1024 with 64.  Us an iteration, 512 / 1024:
+// Ackley 20011 x 30 3.9 / 4.3, Rastrigin 10007 x 25 2.6 / 3.1, 10000 x 100 5.0 /
+// 5.4, Rosenbrock 65536 x 10 3.5 / 3.9, but sphere 100003 x 20 (658 particles a
+// block) 5.65 / 5.5, Rastrigin 250000 x 10 (1645) 10.1 / 8.9.
+constexpr int kResidentThreads = 512;
 constexpr int kResidentMaxThreads = 1024;
 // polls of one word before a wait gives up: each is at least an L2 round trip
 // (several hundred cycles), so seconds -- no exchange takes milliseconds
 constexpr unsigned int kResidentPollLimit = 1u << 23;
-constexpr int kResidentUserThreads = 512;  // 128 registers for a user objective
 
 // shared memory of a block: bounds (float4 per pair), g (float2 per pair),
 // x, v, pbest (float2 per pair and particle), the moved terms, pcost, flags
@@ -182,8 +187,9 @@ __device__ __forceinline__ float coord_get(const float2* A, int d, int p, int ch
 // The run of swarm `s` by the a.blocks blocks that hold it, this one block
 // `rank` of them.  s.flag and s.st may be NULL (a batched swarm): no pending
 // copies, and the global best goes to `result` (cost, index bits, iterations).
-// `prm8`: a user objective's 8 parameters in shared memory.
-template <int OBJ, bool SPLIT, bool CONS>
+// `prm8`: a user objective's 8 parameters in shared memory.  UNROLL: pairs a
+// thread moves between two loop tests.
+template <int OBJ, bool SPLIT, bool CONS, int UNROLL = 1>
 __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams& op, const PhiloxKeys& keys,
                                              const ResidentArgs& a, int rank, float* result = nullptr,
                                              const float* prm8 = nullptr) {
@@ -268,7 +274,7 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
       const bool fl = flag[p] != 0;
       const float2 w2 = dup(w);
       Acc<OBJ, true> acc;
-#pragma unroll 1
+#pragma unroll UNROLL
       for (int j = g0; j < np; j += G) {
         const Rand4 r = pi.draw((uint32_t)j, keys);
         const float2 x = pair_get<ROWS>(X, j, p, chunk);

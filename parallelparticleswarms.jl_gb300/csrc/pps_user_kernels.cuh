@@ -274,7 +274,7 @@ extern "C" __global__ void __launch_bounds__(pps::kUserThreads, PPS_USER_MB4)
 // A whole synchronous run with the state in shared memory (pps_resident.cuh),
 // with or without constraints and however many threads share a particle: one
 // instantiation, since every source pays for its compilation.
-extern "C" __global__ void __launch_bounds__(pps::kResidentUserThreads, 1)
+extern "C" __global__ void __launch_bounds__(pps::kResidentThreads, 1)
     pps_user_resident(pps::SwarmDev s, pps::ObjParams op, pps::PhiloxKeys keys, pps::ResidentArgs a) {
   __shared__ float sp[8];
   pps::user_params(sp, op);
