@@ -40,7 +40,7 @@ __device__ __forceinline__ void async_publish(const SwarmDev& s, unsigned long l
 // The run with every lane's slice exactly S dims (a compile-time count) and
 // the general form's arithmetic in fewer instructions: the draws'
 // loop-invariant rounds carried (PhiloxIteration), the draws' scale in the
-// coefficients (velocity24), a pair's update and cosines in packed f32x2
+// coefficients (draw24), a pair's update and cosines in packed f32x2
 // (pps_pair.cuh), its bounds and g in one 128-bit and one 64-bit load,
 // two-instruction clamps.  Dims past the last are moved as zeros inside [0, 0]
 // and left out of the sums, so a pair needs no branch and the assembler

@@ -445,18 +445,11 @@ __device__ __forceinline__ float velocity(float x, float v, float p, float g, fl
   return __fadd_rn(__fadd_rn(a, b), c);
 }
 
-// The same update from the draws' 24-bit integers m = bits >> 8, with c1s =
-// c1 2^-24 and c2s = c2 2^-24: c1 (m 2^-24) and (c1 2^-24) m are the same
-// real product, so they round to the same value wherever c1s is exact (see
-// coef_scales), and the draw's own multiplication by 2^-24 goes.
+// A draw's 24-bit integer m = bits >> 8, for updates that take c1s = c1 2^-24 and
+// c2s = c2 2^-24 (pps_pair.cuh): c1 (m 2^-24) and (c1 2^-24) m are the same
+// real product, so they round to the same value wherever c1s is exact
+// (coef_scales), and the draw's own multiplication by 2^-24 goes.
 __device__ __forceinline__ float draw24(uint32_t bits) { return __uint2float_rn(bits >> 8); }
-__device__ __forceinline__ float velocity24(float x, float v, float p, float g, float w, float c1s, float c2s,
-                                            uint32_t r1, uint32_t r2) {
-  const float a = __fmul_rn(w, v);
-  const float b = __fmul_rn(__fmul_rn(c1s, draw24(r1)), __fsub_rn(p, x));
-  const float c = __fmul_rn(__fmul_rn(c2s, draw24(r2)), __fsub_rn(g, x));
-  return __fadd_rn(__fadd_rn(a, b), c);
-}
 // whether c 2^-24 is exact (c is 0 or large enough that it stays normal)
 __host__ __device__ inline bool coef_scales(float c) { return c == 0.0f || c >= 0x1p-100f || c <= -0x1p-100f; }
 

@@ -1,6 +1,7 @@
 // pps_pair.cuh -- two dims of a particle per instruction: the update and the
 // cosine objectives' terms in Blackwell's packed f32x2 arithmetic, each lane
-// the scalar operation sequence (velocity24, cos2pi_box), so bit-identical to it.
+// the scalar operation sequence (velocity with draw24, cos2pi_box), so
+// bit-identical to it.
 //
 // The assembler contracts a packed multiply whose only use is a packed add
 // into one fused operation, which rounds once where two operations round
@@ -18,7 +19,8 @@ __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __f
 __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }  // of sums only
 
-// velocity24 of a pair with draw r (r.a, r.b: first dim; r.c, r.d: second)
+// velocity() of a pair with draw r (r.a, r.b: first dim; r.c, r.d: second) and
+// the coefficients times 2^-24
 __device__ __forceinline__ float2 velocity24x2(float2 x, float2 v, float2 p, float2 g, float2 w, float2 c1s, float2 c2s,
                                                const Rand4& r, float2 one, float2 mone) {
   const float2 a = mul(w, v);

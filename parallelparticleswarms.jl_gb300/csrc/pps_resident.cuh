@@ -42,7 +42,7 @@ struct ResidentArgs {
   int iters;
   uint32_t t0;
   float w0, wdamp;
-  float c1s, c2s;     // c1 2^-24, c2 2^-24 (velocity24)
+  float c1s, c2s;     // c1 2^-24, c2 2^-24 (draw24)
   int from_position;
   uint32_t seq0;      // sequence number before the first exchange
   unsigned int poll_limit;
