@@ -278,7 +278,10 @@ __global__ void __launch_bounds__(kPipeWarps * 32) k_step_tsit5_pipe(SwarmDev s,
 
 // The step of an adaptive Tsit5 fit with L lanes per particle: all take every
 // step, each evaluates every L-th save (tsit5a_loss), so a swarm too small for one
-// particle per thread to fill the schedulers gets L times the warps.
+// particle per thread to fill the schedulers gets L times the warps.  Lanes past
+// the last particle (whole groups of L) go straight to the publication: one
+// that followed a real particle would read it while its own lanes, in another
+// warp, write it.
 template <int MODEL, int L>
 __global__ void __launch_bounds__(kOdeThreads) k_step_tsit5a_lanes(SwarmDev s, OdeCfg cfg,
                                                                 const float* __restrict__ data_g, uint64_t seed,
@@ -291,27 +294,29 @@ __global__ void __launch_bounds__(kOdeThreads) k_step_tsit5a_lanes(SwarmDev s, O
   const float* data = ode_observations<kOdeTsit5Adaptive>(cfg);
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L;
   const bool lead = (threadIdx.x & (L - 1)) == 0, valid = i < s.n;
-  const int64_t il = valid ? i : s.n - 1;  // lanes past the last particle follow it and write nothing
-  const Rand4 r0 = philox4x32_10((uint32_t)il, 0u, t, kTagStep, (uint32_t)seed, (uint32_t)(seed >> 32));
-  const Rand4 r1 = philox4x32_10((uint32_t)il, 1u, t, kTagStep, (uint32_t)seed, (uint32_t)(seed >> 32));
-  const float ra[4] = {u01(r0.a), u01(r0.c), u01(r1.a), u01(r1.c)};  // r1 draws of dims 0..3
-  const float rb[4] = {u01(r0.b), u01(r0.d), u01(r1.b), u01(r1.d)};  // r2 draws
-  const bool pending = s.flag[il] != 0;
-  float x[kOdeMaxDim], v[kOdeMaxDim], p[kOdeMaxDim];
+  bool pending = false;
+  float x[kOdeMaxDim] = {}, v[kOdeMaxDim] = {}, p[kOdeMaxDim] = {};
+  float pc0 = 0.0f, c = 0.0f;
+  if (valid) {
+    const Rand4 r0 = philox4x32_10((uint32_t)i, 0u, t, kTagStep, (uint32_t)seed, (uint32_t)(seed >> 32));
+    const Rand4 r1 = philox4x32_10((uint32_t)i, 1u, t, kTagStep, (uint32_t)seed, (uint32_t)(seed >> 32));
+    const float ra[4] = {u01(r0.a), u01(r0.c), u01(r1.a), u01(r1.c)};  // r1 draws of dims 0..3
+    const float rb[4] = {u01(r0.b), u01(r0.d), u01(r1.b), u01(r1.d)};  // r2 draws
+    pending = s.flag[i] != 0;
 #pragma unroll
-  for (int d = 0; d < kOdeMaxDim; ++d) {
-    x[d] = v[d] = p[d] = 0.0f;
-    if (d < D) {
-      const int64_t o = (int64_t)d * s.npad + il;
-      const float xd = s.X[o];
-      p[d] = pending ? xd : s.P[o];
-      v[d] = velocity(xd, s.V[o], p[d], s.g[d], w, c1, c2, ra[d], rb[d]);
-      x[d] = clamp_lb_ub(__fadd_rn(xd, v[d]), s.lb[d], s.ub[d]);
+    for (int d = 0; d < kOdeMaxDim; ++d) {
+      if (d < D) {
+        const int64_t o = (int64_t)d * s.npad + i;
+        const float xd = s.X[o];
+        p[d] = pending ? xd : s.P[o];
+        v[d] = velocity(xd, s.V[o], p[d], s.g[d], w, c1, c2, ra[d], rb[d]);
+        x[d] = clamp_lb_ub(__fadd_rn(xd, v[d]), s.lb[d], s.ub[d]);
+      }
     }
+    pc0 = s.pcost[i];
+    c = tsit5a_loss<MODEL, L>(x, cfg, data);
   }
-  const float pc0 = s.pcost[il];
-  const float c = tsit5a_loss<MODEL, L>(x, cfg, data);
-  __syncwarp();  // every lane has read the particle
+  __syncwarp();  // every lane of the particle, all in one warp, has read it
   unsigned long long key = ~0ull;
   if (valid && lead) {
 #pragma unroll
