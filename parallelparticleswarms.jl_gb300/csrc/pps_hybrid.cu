@@ -39,12 +39,12 @@
 namespace pps {
 
 // the kernels of the registered objectives over the shared device code
-template <int OBJ, int MAXD, bool SMEM>
+template <int OBJ, int MAXD, bool SMEM, bool BOX>
 __global__ void __launch_bounds__(SMEM ? kLbfgsThreads : 128)
     k_lbfgs(const float* __restrict__ X0, int64_t ld, int64_t n, ObjParams op, const float* __restrict__ lbp,
             const float* __restrict__ ubp, LocalOpts o, float* __restrict__ xout, float* __restrict__ fout,
             float* __restrict__ itout, unsigned int* next) {
-  lbfgs_run<OBJ, MAXD, SMEM>(X0, ld, n, op, lbp, ubp, o, xout, fout, itout, next);
+  lbfgs_run<OBJ, MAXD, SMEM, BOX>(X0, ld, n, op, lbp, ubp, o, xout, fout, itout, next);
 }
 
 template <int OBJ, int MAXD, bool SMEM>
@@ -158,22 +158,33 @@ static unsigned resident_blocks(K kernel, int threads, size_t smem, int sm_count
   return (unsigned)(need < resident ? need : resident);
 }
 
-template <int OBJ, int MAXD>
-static int launch_local_lbfgs(pps_swarm* s, const float* x0, const LocalOpts& o, const LocalBufs& b) {
+template <int OBJ, int MAXD, bool BOX>
+static int launch_lbfgs(pps_swarm* s, const float* x0, const LocalOpts& o, const LocalBufs& b) {
   const int64_t n = s->dv.n;
   PPS_CUDA(cudaMemsetAsync(&b.slot->next, 0, sizeof(b.slot->next), s->stream));
   if constexpr (MAXD <= 16) {
     const size_t smem = sizeof(float) * lbfgs_hist_floats(o.history, MAXD) * kLbfgsThreads;
-    PPS_CUDA(cudaFuncSetAttribute(k_lbfgs<OBJ, MAXD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned blocks = resident_blocks(k_lbfgs<OBJ, MAXD, true>, kLbfgsThreads, smem, s->sm_count, n);
-    k_lbfgs<OBJ, MAXD, true><<<blocks, kLbfgsThreads, smem, s->stream>>>(x0, s->dv.npad, n, s->op, s->dv.lb,
-                                                                          s->dv.ub, o, b.x, b.f, b.it, &b.slot->next);
+    const auto kernel = k_lbfgs<OBJ, MAXD, true, BOX>;
+    PPS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned blocks = resident_blocks(kernel, kLbfgsThreads, smem, s->sm_count, n);
+    kernel<<<blocks, kLbfgsThreads, smem, s->stream>>>(x0, s->dv.npad, n, s->op, s->dv.lb, s->dv.ub, o, b.x, b.f, b.it,
+                                                       &b.slot->next);
   } else {
-    const unsigned blocks = resident_blocks(k_lbfgs<OBJ, MAXD, false>, 128, 0, s->sm_count, n);
-    k_lbfgs<OBJ, MAXD, false><<<blocks, 128, 0, s->stream>>>(x0, s->dv.npad, n, s->op, s->dv.lb, s->dv.ub, o, b.x,
-                                                              b.f, b.it, &b.slot->next);
+    const auto kernel = k_lbfgs<OBJ, MAXD, false, BOX>;
+    const unsigned blocks = resident_blocks(kernel, 128, 0, s->sm_count, n);
+    kernel<<<blocks, 128, 0, s->stream>>>(x0, s->dv.npad, n, s->op, s->dv.lb, s->dv.ub, o, b.x, b.f, b.it,
+                                          &b.slot->next);
   }
   return PPS_OK;
+}
+
+// the bounded cosines where the bounds allow them; the widest form has none
+template <int OBJ, int MAXD>
+static int launch_local_lbfgs(pps_swarm* s, const float* x0, const LocalOpts& o, const LocalBufs& b) {
+  if constexpr ((OBJ == kRastrigin || OBJ == kAckley) && MAXD < 64) {
+    if (box_cosines(OBJ, s->op, s->dv.dim, s->host_lb, s->host_ub)) return launch_lbfgs<OBJ, MAXD, true>(s, x0, o, b);
+  }
+  return launch_lbfgs<OBJ, MAXD, false>(s, x0, o, b);
 }
 
 // Broyden: from 8 dims the inverse Jacobian (MAXD^2 floats a particle) lives
@@ -215,10 +226,7 @@ static int launch_local_obj(pps_swarm* s, int kind, const float* x0, const Local
   if constexpr (OBJ >= kBeale) {  // closed forms are defined for dim <= 2
     rc = launch_local_t<OBJ, 2>(s, kind, x0, o, b);
   } else {
-    // the cosines' bounded form needs moderate bounds; others take the widest kernel
-    const bool wide = kind == 0 && !box_cosines(OBJ, s->op, D, s->host_lb, s->host_ub);
-    if (wide) rc = launch_local_lbfgs<OBJ, 64>(s, x0, o, b);
-    else if (D <= 2) rc = launch_local_t<OBJ, 2>(s, kind, x0, o, b);
+    if (D <= 2) rc = launch_local_t<OBJ, 2>(s, kind, x0, o, b);
     else if (D <= 4) rc = launch_local_t<OBJ, 4>(s, kind, x0, o, b);
     else if (D <= 8) rc = launch_local_t<OBJ, 8>(s, kind, x0, o, b);
     else if (D <= 10) rc = kind == 0 ? launch_local_lbfgs<OBJ, 10>(s, x0, o, b)

@@ -60,14 +60,12 @@ struct LbfgsHistory<MAXD, false> {
 // floats of shared memory one thread's L-BFGS history takes
 __host__ __device__ constexpr size_t lbfgs_hist_floats(int m, int maxd) { return (size_t)2 * m * maxd + 2 * (size_t)m; }
 
-// The forms up to 32 dims take the cosines of bounded arguments (cos2pi_box);
-// bounds beyond its limit run in the widest form (launch_local_obj).  With the
-// gradient taken from the accepted point's own sums instead of a second
+// BOX: the cosines' arguments stay below cos2pi_box's limit (box_cosines; every
+// point is clamped into the bounds).  Bounds beyond it, none at all among them,
+// take the same forms with BOX off.  With the gradient taken from the accepted point's own sums instead of a second
 // evaluation, 65,536 x 10-D Ackley after 100 iterations went from 8.5 to 7.0 ms,
 // Rastrigin from 3.6 to 3.1.  (Line searches cut into bursts, so that lanes with
 // short ones go on: 12 to 15 ms -- most lanes search long at the same time.)
-__host__ __device__ constexpr bool lbfgs_box(int maxd) { return maxd < 64; }
-
 // One L-BFGS per particle.  With `next` NULL each thread runs particle
 // blockIdx.x * blockDim.x + threadIdx.x.  With a work counter `next` (zero at
 // launch) the grid is the resident threads, and a thread whose particle has
@@ -76,13 +74,12 @@ __host__ __device__ constexpr bool lbfgs_box(int maxd) { return maxd < 64; }
 // would otherwise run until its slowest particle stops while the other lanes
 // idle.  Either way a particle's operations are the same, so its result does
 // not depend on the thread that computes it.
-template <int OBJ, int MAXD, bool SMEM>
+template <int OBJ, int MAXD, bool SMEM, bool BOX = false>
 __device__ __forceinline__ void lbfgs_run(const float* __restrict__ X0, int64_t ld, int64_t n, const ObjParams& op,
                                           const float* __restrict__ lbp, const float* __restrict__ ubp,
                                           const LocalOpts& o, float* __restrict__ xout, float* __restrict__ fout,
                                           float* __restrict__ itout, unsigned int* next = nullptr) {
   extern __shared__ float hist_sm[];
-  constexpr bool BOX = lbfgs_box(MAXD);  // every point is clamped into the bounds
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int D = op.dim;
