@@ -62,7 +62,9 @@ __host__ __device__ constexpr size_t lbfgs_hist_floats(int m, int maxd) { return
 
 // BOX: the cosines' arguments stay below cos2pi_box's limit (box_cosines; every
 // point is clamped into the bounds).  Bounds beyond it, none at all among them,
-// take the same forms with BOX off.  With the gradient taken from the accepted point's own sums instead of a second
+// take the same forms with BOX off (20,000 particles, 50 iterations, us: Ackley
+// 2-D 655, 10-D 1061, 24-D 9411, Rastrigin 10-D 803; the 64-dim kernel takes 27,000 to
+// 31,000 for any of them).  With the gradient taken from the accepted point's own sums instead of a second
 // evaluation, 65,536 x 10-D Ackley after 100 iterations went from 8.5 to 7.0 ms,
 // Rastrigin from 3.6 to 3.1.  (Line searches cut into bursts, so that lanes with
 // short ones go on: 12 to 15 ms -- most lanes search long at the same time.)
