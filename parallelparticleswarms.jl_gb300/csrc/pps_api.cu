@@ -561,9 +561,18 @@ static int sync_like_run(pps_swarm* s, int32_t maxiters, float w, float wdamp, f
         PPS_CUDA(cudaMemcpyAsync(&status, &s->dv.st->status, sizeof(status), cudaMemcpyDeviceToHost, s->stream));
       PPS_CUDA(cudaStreamSynchronize(s->stream));
       if ((rc = finish_timing(s, device_ms))) return rc;
+      if (status & kStatusResidentTimeout) {
+        // some blocks may have written their state back and others not: the
+        // swarm needs a new start, and the next run a clear bit
+        s->initialized = 0;
+        s->local_valid = 0;
+        status &= ~kStatusResidentTimeout;
+        PPS_CUDA(cudaMemcpyAsync(&s->dv.st->status, &status, sizeof(status), cudaMemcpyHostToDevice, s->stream));
+        PPS_CUDA(cudaStreamSynchronize(s->stream));
+        return set_error(PPS_ETIMEOUT,
+                         "the resident run timed out waiting for another block's best (call pps_swarm_init to start over)");
+      }
       s->t += (uint32_t)maxiters;
-      if (status & kStatusResidentTimeout)
-        return set_error(PPS_ETIMEOUT, "the resident run timed out waiting for another block's best");
       return PPS_OK;
     }
   }

@@ -1023,6 +1023,7 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
   int dev = -1;
   cudaGetDevice(&dev);
   if (dev != b->device) PPS_CUDA(cudaSetDevice(b->device));
+  b->ran = false;  // no results until this run's are complete
   int rc = prepare(b);
   if (rc) return rc;
   const int ns = (int)b->descs.size();

@@ -21,7 +21,7 @@
 // 52 / 18, this form 50 / 17.
 //
 // The grid is cooperative, so a team may wait for the others of its fit; a
-// wait that gives up (kOdeTeamLooks looks) sets the run's error word.  Positions,
+// wait that gives up (`looks` looks) sets the run's error word.  Positions,
 // velocities, personal bests and costs pass between SMs through L2: written
 // before a device fence and the phase's counter, read past L1.  Each fit's
 // result equals its solve alone, bit for bit (Philox by particle, the argmin
@@ -178,11 +178,11 @@ __device__ __forceinline__ void ode_unit(const BatchSwarm& sw, OdeCtl* c, unsign
 
 // units: every team's units, team by team (teams of block b: b teams .. b teams
 // + teams - 1), offsets[team] .. offsets[team + 1]; next: each unit's next phase
-// (zero at launch).  `one` is a run-time 1.0f (ode_loss2).
+// (zero at launch); looks: kOdeTeamLooks.  `one` is a run-time 1.0f (ode_loss2).
 template <bool PACK>
 __global__ void __launch_bounds__(kTeam* kMaxTeams, 1)
     k_ode_teams(const BatchSwarm* __restrict__ descs, const OdeUnit* __restrict__ units, const int* __restrict__ offsets,
-                unsigned int* next, OdeCtl* ctl, int nfits, int data_floats, float one) {
+                unsigned int* next, OdeCtl* ctl, int nfits, int data_floats, unsigned int looks, float one) {
   extern __shared__ float obs[];
   __shared__ unsigned long long red_s[kMaxTeams][kTeam / 32];
   __shared__ int pick_s[kMaxTeams][2];
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kTeam* kMaxTeams, 1)
     if (tid < 32) {
       // the next of the team's units whose phase is open, from the one after the last
       int got = -1;
-      for (unsigned int look = 0; look < kOdeTeamLooks && got < 0; ++look) {
+      for (unsigned int look = 0; look < looks && got < 0; ++look) {
         for (int base = 0; base < count && got < 0; base += 32) {
           int e = at + base + tid;
           bool ready = false;
@@ -353,7 +353,7 @@ int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSw
   cfg.attrs = at;
   cfg.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ddescs, (const OdeUnit*)du, (const int*)doff, next, ctl, nf,
-                                           data_floats, 1.0f);
+                                           data_floats, wait_polls(kOdeTeamLooks), 1.0f);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();
     return PPS_OK;

@@ -11,6 +11,8 @@
 // line is the shared memory of all SMs (about 2.8 M coordinates of 12 bytes,
 // 2.1 M with the moved terms): beyond it the state has to stream from L2 or
 // memory each iteration, which k_sync_step does.
+#include <cstdlib>
+
 #include "pps_internal.h"
 #include "pps_resident.cuh"
 
@@ -32,6 +34,13 @@ constexpr int64_t kResidentCoords = 256;     // coordinates a block of several h
 constexpr int kResidentMinBlocks = 16;
 
 static bool terms_moved(int objective) { return objective == kRastrigin || objective == kAckley; }
+
+unsigned int wait_polls(unsigned int usual) {
+  const char* e = getenv("PPS_WAIT_POLLS");
+  if (!e || *e < '0' || *e > '9') return usual;
+  const unsigned long n = strtoul(e, nullptr, 10);
+  return n < usual ? (unsigned int)n : usual;
+}
 
 // bytes of the exchange words the swarm's run needs (0: none)
 size_t resident_exchange_bytes(int objective, int dim, int64_t n, int ncons, int sm_count) {
@@ -152,7 +161,7 @@ int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w,
   a.c2s = c2 * 0x1p-24f;
   a.from_position = from_position;
   a.seq0 = s->xch_seq;
-  a.poll_limit = kResidentPollLimit;
+  a.poll_limit = wait_polls(kResidentPollLimit);
   a.one = 1.0f;
   a.xch = s->xch_dev;
   a.status = &s->dv.st->status;
@@ -164,7 +173,7 @@ int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w,
     cudaFuncAttributes fa;
     PPS_CUDA(cudaFuncGetAttributes(&fa, kernel));
     if (fa.sharedSizeBytes > kResidentStatic) return PPS_OK;  // the source's own shared memory leaves no room
-    a.poll_limit = kResidentUserPollLimit;
+    a.poll_limit = wait_polls(kResidentUserPollLimit);
     rc = launch_one(kernel, s, p, keys, a, taken);
     if (*taken) s->xch_seq += (uint32_t)iters;
     return rc;
