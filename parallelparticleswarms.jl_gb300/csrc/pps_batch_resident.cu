@@ -262,6 +262,7 @@ int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vect
       j.a.wdamp = d.wdamp;
       j.a.c1s = d.c1 * 0x1p-24f;
       j.a.c2s = d.c2 * 0x1p-24f;
+      j.a.start_limit = kResidentStartLimit;
       j.a.poll_limit = wait_polls(kResidentPollLimit);
       j.a.one = 1.0f;
       j.result = d.result;

@@ -100,8 +100,8 @@ int sync_bulk_prepare(pps_swarm* s, int* blocks_per_sm);
 int check_device_status(pps_swarm* s);
 int launch_sync_step_bulk(pps_swarm* s, float c1, float c2, bool* taken);
 bool sync_bulk_requested();  // PPS_SYNC_KERNEL=bulk
-// the polls after which a wait between blocks gives up: `usual`, or fewer with
-// PPS_WAIT_POLLS=<n> (read at each launch; 0 lets every such wait run out)
+// the polls after which a wait between running blocks gives up: `usual`, or fewer
+// with PPS_WAIT_POLLS=<n> (read at each launch; 0 lets every such wait run out)
 unsigned int wait_polls(unsigned int usual);
 // a whole run in one launch with the state in shared memory (pps_resident.cu)
 struct ResidentPlan {

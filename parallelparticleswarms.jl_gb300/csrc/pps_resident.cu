@@ -24,8 +24,6 @@ __global__ void __launch_bounds__(T, 1)
   resident_run<OBJ, SPLIT, CONS>(s, op, keys, a, (int)blockIdx.x);
 }
 
-// a user objective may take its own time, and unevenly: minutes
-constexpr unsigned int kResidentUserPollLimit = 1u << 29;
 constexpr size_t kResidentSmem = 227u << 10;  // a block's shared memory, static part included
 constexpr size_t kResidentStatic = 2048;
 constexpr int kResidentMaxDim = 1024;  // g and bounds of more dims crowd the state out
@@ -161,6 +159,7 @@ int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w,
   a.c2s = c2 * 0x1p-24f;
   a.from_position = from_position;
   a.seq0 = s->xch_seq;
+  a.start_limit = kResidentStartLimit;
   a.poll_limit = wait_polls(kResidentPollLimit);
   a.one = 1.0f;
   a.xch = s->xch_dev;
@@ -173,7 +172,7 @@ int launch_resident(pps_swarm* s, const ResidentPlan& p, int32_t iters, float w,
     cudaFuncAttributes fa;
     PPS_CUDA(cudaFuncGetAttributes(&fa, kernel));
     if (fa.sharedSizeBytes > kResidentStatic) return PPS_OK;  // the source's own shared memory leaves no room
-    a.poll_limit = wait_polls(kResidentUserPollLimit);
+    a.poll_limit = wait_polls(kResidentStartLimit);
     rc = launch_one(kernel, s, p, keys, a, taken);
     if (*taken) s->xch_seq += (uint32_t)iters;
     return rc;

@@ -27,7 +27,10 @@
 // A user objective (kUserObjective, compiled by NVRTC) reads the new position
 // back through its accessor, so its state lies at [dim][particle]; the
 // read-back is from shared memory instead of L2.
-// The wait for a post is bounded (poll_limit polls); a wait that gives up sets
+// The wait for a post is bounded: poll_limit polls, and start_limit in the first
+// exchange: a cooperative launch promises that the blocks can all be resident,
+// not that they start together while other work holds SMs (on a GB300 they did,
+// beside a batch of fits and beside an async run of a second).  A wait that gives up sets
 // IterState::status bit 3 and the block leaves the loop.
 #pragma once
 #include "pps_pair.cuh"
@@ -45,7 +48,8 @@ struct ResidentArgs {
   float c1s, c2s;     // c1 2^-24, c2 2^-24 (draw24)
   int from_position;
   uint32_t seq0;      // sequence number before the first exchange
-  unsigned int poll_limit;
+  unsigned int start_limit;  // polls of the first exchange
+  unsigned int poll_limit;   // polls of the others
   float one;          // 1.0f (pps_pair.cuh)
   unsigned long long* xch;  // exchange of several blocks: two buffers of resident_words
   unsigned int* status;     // a wait that gives up sets kStatusResidentTimeout here
@@ -63,8 +67,12 @@ constexpr bool kTermsMoved = OBJ == kRastrigin || OBJ == kAckley;
 constexpr int kResidentThreads = 512;
 constexpr int kResidentMaxThreads = 1024;
 // polls of one word before a wait gives up: each is at least an L2 round trip
-// (several hundred cycles), so seconds -- no exchange takes milliseconds
+// (several hundred cycles), so seconds -- between blocks that all run, no
+// exchange takes milliseconds
 constexpr unsigned int kResidentPollLimit = 1u << 23;
+// the first exchange of a launch, and every one of a user objective, which may
+// take its own time and unevenly: minutes
+constexpr unsigned int kResidentStartLimit = 1u << 29;
 
 // shared memory of a block: bounds (float4 per pair), g (float2 per pair),
 // x, v, pbest (float2 per pair and particle), the moved terms, pcost, flags
@@ -355,6 +363,7 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     if (!none) src = (a.from_position || flag[lp]) ? X : P;
     // ---- agree on the global best
     const uint32_t seq = a.seq0 + 1u + (uint32_t)it;
+    const unsigned int limit = it == 0 ? a.start_limit : a.poll_limit;
     const int nb = a.blocks;
     unsigned long long* kw = a.xch + (size_t)par * resident_words(nb, D);  // keys
     unsigned long long* vw = kw + 2 * (size_t)nb;                          // vectors
@@ -373,14 +382,14 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     }
     if (nb > 1 && warp == 0) {
       bool ok = true;
-      const unsigned long long k = await_keys(kw, nb, seq, a.poll_limit, &ok);
+      const unsigned long long k = await_keys(kw, nb, seq, limit, &ok);
       ok = __all_sync(0xffffffffu, ok);
       // nobody's personal best beat the last global best: its vector stands
       if (ok && (a.from_position || !have_prev || k != prev)) {
         const unsigned long long* v = vw + (size_t)((int64_t)(uint32_t)k / chunk) * D;
         for (int d = lane; d < D && ok; d += 32) {
           uint32_t bits = 0u;
-          ok = await_word(v + d, seq, a.poll_limit, &bits);
+          ok = await_word(v + d, seq, limit, &bits);
           gs[d] = __uint_as_float(bits);
         }
         ok = __all_sync(0xffffffffu, ok);
