@@ -525,12 +525,25 @@ int launch_init_ode(pps_swarm* s, int sampler, const float* u0_dev) {
   return PPS_OK;
 }
 
-// Lanes per particle of an adaptive fit: eight up to the size at which the
-// extra steps cost what the spread saves gain (LV, us an iteration, 1 / 4 / 8
-// lanes: 500 particles 110 / 95 / 68, 10000 130 / 115 / 94, 20000 140 / 126 / 121,
-// 40000 146 / 177 / 179; FHN 10000 75 / 66 / 42, 40000 111 / 125 / 100).
-constexpr int64_t kAdaptiveLanesMaxN = 24000;
+// Whether an adaptive fit takes eight lanes per particle.  All lanes take every
+// step and share the saves, so it pays where the saves are most of the work,
+// and the more particles there are to fill the schedulers the more of it they
+// have to be.  One thread / eight lanes, us an iteration, the worse of LV and FHN
+// at tolerances 1e-3 and 1e-6 (30 first steps on [0, 3]): 301 saves 500 particles
+// 110 / 68, 10000 130 / 94, 24000 0.96 of one thread's time; 201 saves 20000
+// 0.99; 101 saves 12000 0.99, 16000 1.18; 61 saves 4000 1.00, 10000 1.07; 41 saves
+// 500 1.11; 16 saves 24000 1.91.  So up to kLanesAnyDensity particles 64 saves
+// suffice; beyond, a first step has to hold particles / 2400 saves, at
+// tolerances that keep the steps near the first one's length.
 constexpr int kAdaptiveLanes = 8;
+constexpr int kLanesMinSaves = 64;
+constexpr int64_t kLanesAnyDensity = 4000, kLanesPerDensity = 2400, kLanesMaxN = 24000;
+
+static bool adaptive_lanes(const OdeCfg& c, int64_t n) {
+  if (c.method != kOdeTsit5Adaptive || c.nsaves < kLanesMinSaves || n > kLanesMaxN) return false;
+  if (n <= kLanesAnyDensity) return true;
+  return c.rtol >= 1e-6f && (double)c.dt * kLanesPerDensity >= 0.999 * (double)c.save_dt * (double)n;
+}
 
 // Steps per chunk of the pipelined fixed-step form, 0 where it does not apply:
 // a swarm that fills the GPU with one particle per thread (us an iteration of
@@ -578,7 +591,7 @@ int launch_sync_step_ode(pps_swarm* s, float c1, float c2) {
     PPS_CUDA(cudaGetLastError());
     return PPS_OK;
   }
-  if (c.method == kOdeTsit5Adaptive && s->dv.n <= kAdaptiveLanesMaxN) {
+  if (adaptive_lanes(c, s->dv.n)) {
     constexpr int L = kAdaptiveLanes;
     const unsigned blocks = (unsigned)((s->dv.n * L + kOdeThreads - 1) / kOdeThreads);
     if (lv)

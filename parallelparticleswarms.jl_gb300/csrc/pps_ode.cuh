@@ -468,7 +468,8 @@ __device__ __forceinline__ float tsit5a_loss(const float* p, const OdeCfg& c, co
           tm = __fmul_rn(__int2float_rn(m), c.save_dt);
         }
       } else {
-        for (int cnt = L; cnt == L && m < c.nsaves; m += cnt) {
+        const bool any = __fmul_rn(__int2float_rn(m), c.save_dt) <= tn1;  // the same in all lanes
+        for (int cnt = any ? L : 0; cnt == L && m < c.nsaves; m += cnt) {
           const int mm = m + lane;
           const float tmm = __fmul_rn(__int2float_rn(mm), c.save_dt);
           const bool in = mm < c.nsaves && tmm <= tn1;

@@ -16,10 +16,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 3, 17, 31, 113])
 def test_ragged_swarms(pps, orc, model, n):
     from parallelparticleswarms import ode
-    obs = np.random.default_rng(n).uniform(0.2, 2.0, (41, 2)).astype(np.float32)
+    obs = np.random.default_rng(n).uniform(0.2, 2.0, (81, 2)).astype(np.float32)
     make = ode.lv_problem if model == "lv" else ode.fhn_problem
     prob = ode.adaptive(make(obs, u0=(1.0, 1.0), dt=0.1, nsteps=30, save_every=1, lb=0.0, ub=3.0, method="tsit5",
-                             save_dt=0.05))
+                             save_dt=0.0375))
     with pps.Swarm(prob, n, seed=6) as sw:
         sw.init()
         ref = orc.OracleSwarm(oracle_ode_problem(orc, prob), n, 6).init()
