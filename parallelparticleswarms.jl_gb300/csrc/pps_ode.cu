@@ -545,21 +545,46 @@ static bool adaptive_lanes(const OdeCfg& c, int64_t n) {
   return c.rtol >= 1e-6f && (double)c.dt * kLanesPerDensity >= 0.999 * (double)c.save_dt * (double)n;
 }
 
-// Steps per chunk of the pipelined fixed-step form, 0 where it does not apply:
-// a swarm that fills the GPU with one particle per thread (us an iteration of
-// 30 steps and 301 saves, one thread / pipeline: 500 particles 28.6 / 12.7,
-// 10000 29.3 / 16.8, 20000 31.3 / 25.6, 40000 35.7 / 39.7), fewer than two
-// saves a step (no dense output to take off the chain), more steps or saves a
-// chunk than it holds.  The save table's steps are found as the kernel finds
-// them.
-constexpr int64_t kPipeMaxN = 28000;
+// Where the pipelined fixed-step form pays.  What it takes off the chain are the
+// saves, what it adds is a fixed part (the table in every block, chunks of one
+// warp after the other) and, on large swarms, blocks that do not all fit the SMs
+// at once: 32 particles need 52 kB and more.  Its time relative to one thread a
+// particle, the worse of LV and FHN (steps x saves a step at particles): 30 x 10 at
+// 500 / 10000 / 20000 0.48 / 0.57 / 0.78, 4 x 10 at 500 1.16, 12 x 10 0.81, 24 x 3 at
+// 10000 0.97, 24 x 2 1.07, 400 x 2 at 10000 (two rounds of blocks) 1.03, 30 x 3 at
+// 15000 / 20000 0.98 / 1.09, 400 x 5 at 15000 (four rounds) 1.19, 18 x 10 at
+// 24000 / 28000 0.95 / 1.05, 30 x 10 at 28000 0.89.  Each row: up to so many
+// particles, from so many saves, saves a step and steps on, and at most so many
+// rounds of resident blocks.
+struct PipeRow {
+  int64_t n;
+  int saves, ratio, steps, rounds;
+};
+constexpr PipeRow kPipeRows[] = {
+    {10240, 72, 2, 4, 1}, {10240, 72, 3, 4, 2}, {16000, 90, 3, 4, 2}, {24000, 180, 5, 12, 3}, {28000, 300, 10, 12, 3}};
 
-static int pipe_chunk(const OdeCfg& c, int64_t particles) {
-  if (c.method != kOdeTsit5 || particles > kPipeMaxN || c.nsteps > kPipeMaxSteps ||
-      c.nsaves < 2 * (int64_t)c.nsteps)
-    return 0;
+static bool pipe_pays(const OdeCfg& c, int64_t particles, size_t smem, int sm_count) {
+  // blocks of 256 threads with 64 registers: four an SM, fewer by shared memory (228 kB, 1 kB of it a block's own)
+  int64_t per_sm = (int64_t)((228u << 10) / (smem + 1024));
+  per_sm = per_sm > 4 ? 4 : per_sm;
+  const int64_t blocks = (particles + 31) / 32, wave = per_sm * sm_count;
+  const int64_t rounds = (blocks + wave - 1) / wave;
+  if (rounds > per_sm + 1) return false;  // few blocks an SM hide little: 400 x 10 at 10000 (three rounds of one) 1.08
+  for (const PipeRow& r : kPipeRows)
+    if (particles <= r.n && c.nsaves >= r.saves && c.nsaves >= (int64_t)r.ratio * c.nsteps && c.nsteps >= r.steps &&
+        rounds <= r.rounds)
+      return true;
+  return false;
+}
+
+// Steps per chunk of the pipelined form, 0 where it is not taken: where it does
+// not pay, or a solve has more steps, or a chunk more saves, than it holds.  The
+// save table's steps are found as the kernel finds them.
+static int pipe_chunk(const OdeCfg& c, int64_t particles, int sm_count) {
+  if (c.method != kOdeTsit5 || c.nsteps > kPipeMaxSteps || c.nsaves < 2 * (int64_t)c.nsteps) return 0;
   for (int K : {6, 3, 1}) {
-    if (pipe_smem(c.nsaves, c.nsteps, K) > (size_t)kPipeSmemMax) continue;
+    const size_t smem = pipe_smem(c.nsaves, c.nsteps, K);
+    if (smem > (size_t)kPipeSmemMax) continue;
     int most = 0, count = 0, at = 0, n = 0;
     for (int m = 1; m < c.nsaves; ++m) {
       const float tm = (float)m * c.save_dt;
@@ -570,7 +595,7 @@ static int pipe_chunk(const OdeCfg& c, int64_t particles) {
       }
       if (++count > most) most = count;
     }
-    if (most <= kPipeMaxSaves) return K;
+    if (most <= kPipeMaxSaves) return pipe_pays(c, particles, smem, sm_count) ? K : 0;
   }
   return 0;
 }
@@ -579,7 +604,7 @@ int launch_sync_step_ode(pps_swarm* s, float c1, float c2) {
   const OdeCfg c = cfg_of(s);
   const int from_pos = (s->flags & PPS_FLAG_GBEST_FROM_POSITION) ? 1 : 0;
   const bool lv = s->objective == kLvFit;
-  if (const int K = pipe_chunk(c, s->dv.n)) {
+  if (const int K = pipe_chunk(c, s->dv.n, s->sm_count)) {
     const unsigned blocks = (unsigned)((s->dv.n + 31) / 32);
     const size_t smem = pipe_smem(c.nsaves, c.nsteps, K);
     if (lv)

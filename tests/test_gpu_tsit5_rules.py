@@ -46,3 +46,21 @@ def test_adaptive_lines(pps, orc, saves, n):
 def test_adaptive_few_saves_time(pps, model, saves):
     prob = _fit(pps, model, 30, saves, adaptive=True)
     assert _time(pps, prob, 24000) <= 1.2 * _time(pps, prob, 24320)
+
+
+# (steps, saves, particles): the first and the last of each row of the rule, and its neighbours
+FIXED = [(4, 71, 40), (4, 72, 40), (3, 72, 40), (36, 72, 10240), (36, 72, 10241), (24, 90, 10241), (24, 90, 16001),
+         (12, 180, 24000), (12, 180, 24001), (12, 300, 28000), (12, 300, 28001), (400, 801, 10000), (150, 900, 12000), (8, 700, 33), (12, 301, 33),
+         (13, 111, 33)]
+
+
+@pytest.mark.parametrize("steps,saves,n", FIXED)
+def test_fixed_step_lines(pps, orc, steps, saves, n):
+    _same(pps, orc, _fit(pps, "lv", steps, saves), n)
+
+
+@pytest.mark.parametrize("model", ["lv", "fhn"])
+@pytest.mark.parametrize("steps,saves", [(4, 21), (30, 61)])
+def test_fixed_step_few_saves_time(pps, model, steps, saves):
+    prob = _fit(pps, model, steps, saves)
+    assert _time(pps, prob, 28000) <= 1.2 * _time(pps, prob, 28160)
