@@ -533,14 +533,26 @@ static int run_steps(pps_swarm* s, int32_t maxiters, float c1, float c2, uint32_
   return PPS_OK;
 }
 
+// Runs of one iteration (two of a user objective with many particles) whose
+// dims are few stay stepwise: a cooperative launch, the state in and out and a
+// status read cost more than the step saves.  One iteration, us a call, stepwise /
+// resident: sphere 20000 x 2 29.0 / 32.4, 10^6 x 2 39.7 / 46.0, 300000 x 7 40.3 /
+// 44.1, 200000 x 10 38.1 / 43.7, but 65536 x 10 36.1 / 31.6, 100003 x 20 49.1 / 43.9;
+// two: sphere 10^6 x 2 57.9 / 56.9, a user objective there 60.9 / 68.6.
+static bool few_steps(const pps_swarm* s, int32_t maxiters) {
+  if (maxiters > 2) return false;
+  const bool few_dims = s->dv.dim <= 8 || (s->dv.dim <= 16 && s->dv.n > 100000);
+  return few_dims && (maxiters == 1 || (is_user(s->objective) && s->dv.n > 300000));
+}
+
 // whether a run of this swarm keeps its state on chip (pps_resident.cu):
-// the swarm fits, the pair arithmetic is exact for it (pair_form), and the
-// TMA-staged step kernel has not been asked for
-static bool resident_applies(const pps_swarm* s, float c1, float c2, ResidentPlan* plan) {
+// the swarm fits, the pair arithmetic is exact for it (pair_form), the run is
+// long enough, and the TMA-staged step kernel has not been asked for
+static bool resident_applies(const pps_swarm* s, int32_t maxiters, float c1, float c2, ResidentPlan* plan) {
   if (s->shard || !s->owns_memory || !pair_form(s, c1, c2)) return false;
   if (sync_bulk_requested()) return false;
   if (!resident_plan(s->objective, s->dv.dim, s->dv.n, s->dv.ncons, s->sm_count, plan)) return false;
-  return plan->blocks == 1 || s->xch_dev;
+  return plan->blocks == 1 || (s->xch_dev && !few_steps(s, maxiters));
 }
 
 static int sync_like_run(pps_swarm* s, int32_t maxiters, float w, float wdamp, float c1, float c2,
@@ -548,7 +560,7 @@ static int sync_like_run(pps_swarm* s, int32_t maxiters, float w, float wdamp, f
   int rc = check_run(s, maxiters, w, wdamp, c1, c2);
   if (rc) return rc;
   ResidentPlan plan;
-  if (maxiters > 0 && resident_applies(s, c1, c2, &plan)) {
+  if (maxiters > 0 && resident_applies(s, maxiters, c1, c2, &plan)) {
     bool taken = false;
     PPS_CUDA(cudaEventRecord(s->ev0, s->stream));
     if ((rc = launch_resident(s, plan, maxiters, w, wdamp, c1, c2,

@@ -234,8 +234,12 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     flag[p] = s.flag ? s.flag[first + p] : 0;
   }
   if (tid == 0) bail = 0;
-  for (int p = lane; p < cnt; p += 32) {  // a warp per pair row
-    for (int j = warp; j < np; j += nw) {
+  // 32 particles of a pair row at a time, dealt to all warps: rows alone leave
+  // most warps idle where the dims are few (a 2-D swarm has one row)
+  const int tiles = (cnt + 31) >> 5, moves = tiles * np;
+  for (int m = warp; m < moves; m += nw) {
+    const int j = m / tiles, p = ((m - j * tiles) << 5) + lane;
+    if (p < cnt) {
       const int64_t o = (int64_t)(2 * j) * s.npad + first + p;
       const bool two = 2 * j + 1 < D;
       pair_put<ROWS>(X, j, p, chunk, make_float2(s.X[o], two ? s.X[o + s.npad] : 0.0f));
@@ -413,9 +417,10 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
   }
 
   // ---- the state back to global memory, personal bests canonical
-  for (int p = lane; p < cnt; p += 32) {
-    const bool fl = flag[p] != 0;
-    for (int j = warp; j < np; j += nw) {
+  for (int m = warp; m < moves; m += nw) {
+    const int j = m / tiles, p = ((m - j * tiles) << 5) + lane;
+    if (p < cnt) {
+      const bool fl = flag[p] != 0;
       const int64_t o = (int64_t)(2 * j) * s.npad + first + p;
       const float2 x = pair_get<ROWS>(X, j, p, chunk), v = pair_get<ROWS>(V, j, p, chunk);
       const float2 q = fl ? x : pair_get<ROWS>(P, j, p, chunk);
