@@ -619,18 +619,19 @@ size_t batch_smem_bytes(int maxdim, int data_floats, int64_t maxchunk) {
   return sizeof(float) * (3 * (size_t)maxdim + (size_t)data_floats) + (size_t)maxchunk + 64;
 }
 
-// Shape limits: PPS_BATCH_MAX_CLUSTER (1..16, default 4) caps the CTAs a swarm
-// is split over (ODE fits: kOdeMaxCluster), PPS_ODE_THREADS (128..1024, default
-// 128) is the block of an ODE-fit CTA.  They change how work is placed, never
-// what is computed.  Clusters above 8 CTAs are a non-portable size.
+// Shape limits: PPS_BATCH_MAX_CLUSTER (1..16; default 4, ODE fits 4 or 8) caps the
+// CTAs a swarm is split over, PPS_ODE_THREADS (128..1024) is the largest block of
+// an ODE-fit CTA, then sized to half the fit's particles.  They change how work
+// is placed, never what is computed.  Clusters above 8 CTAs are a non-portable
+// size.
 static int env_int(const char* name, int dflt, int lo, int hi) {
   const char* e = getenv(name);
   const int v = e ? atoi(e) : dflt;
   return (v >= lo && v <= hi) ? v : dflt;
 }
-static int max_cluster() {
-  static const int v = env_int("PPS_BATCH_MAX_CLUSTER", 4, 1, 16);
-  return v;
+static int max_cluster(int dflt) {
+  static const int v = env_int("PPS_BATCH_MAX_CLUSTER", 0, 1, 16);
+  return v ? v : dflt;
 }
 // Dims of the reference CTA of the work-based split: a swarm gets one CTA per
 // width particles of kBatchDimRef dims (PPS_BATCH_DIM_REF overrides; 0 splits
@@ -643,24 +644,40 @@ static int batch_dim_ref() {
   static const int v = env_int("PPS_BATCH_DIM_REF", kBatchDimRef, 0, 4096);
   return v;
 }
-static int ode_threads() {
-  static const int v = env_int("PPS_ODE_THREADS", 128, 128, 1024) / 32 * 32;
+static int ode_threads() {  // 0: not given
+  static const int v = env_int("PPS_ODE_THREADS", 0, 128, 1024);
   return v;
 }
-constexpr int kOdeMaxCluster = 8;
+// The shape of an ODE fit's CTAs, two particles per thread and trip (the packed
+// RK4 losses).  CTAs of one warp per scheduler spread a fit over more SMs than few
+// large ones do: 128 fits of 1000 and 2000 steps, 512 threads and clusters of 4:
+// 98 ms, 128 threads and clusters of 8: 58 ms.  But an iteration across a cluster
+// waits 4 us for its barriers, and a trip costs 1 us beside its steps, so short
+// solves keep the large block: us an iteration, large / small, one fit of 512
+// particles and 10 steps 2.2 / 4.8, 60 steps 7.0 / 7.5, 150 steps 15.9 / 12.7; of
+// 1024 and 10 steps 3.7 / 4.6, 30 steps 7.7 / 5.7; of 4096 and 30 steps 11.0 /
+// 11.6, 60 steps 16.8 / 15.0; 64 of 16384 and 10 steps 43 / 52, 30 steps 73 / 82.
+static void ode_shape(const BatchSwarm& d, int* threads, int* cluster) {
+  const int steps = ode_cfg(d.op, d.ndata).nsteps, given = ode_threads();
+  const bool brief = steps < (d.n <= 512 ? 64 : d.n <= 2048 ? 24 : 32);
+  int T = 128;
+  if (brief || given) {
+    const int64_t half = (d.n + 1) / 2;
+    const int most = given ? given : 512;
+    while (T < half && 2 * T <= most) T *= 2;
+  }
+  const int64_t c = (d.n + 2 * (int64_t)T - 1) / (2 * (int64_t)T);
+  const int cmax = max_cluster(brief || given ? 4 : 8);
+  *threads = T;
+  *cluster = (int)(c < cmax ? c : cmax);
+}
 
 LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread) {
   LaunchGroup g{};
-  const int cmax = max_cluster();
+  const int cmax = max_cluster(4);
   if (is_ode(d.objective)) {
     g.kind = 1;
-    // two particles per thread and trip (the packed RK4 losses); CTAs of one
-    // warp per scheduler spread a fit over more SMs than few large ones do
-    // (PPS_ODE_THREADS): 128 mixed fits, 512 threads and clusters of 4: 98 ms,
-    // 128 threads and clusters of 8: 58 ms
-    g.T = ode_threads();
-    const int64_t c = (d.n + 2 * (int64_t)g.T - 1) / (2 * (int64_t)g.T);
-    g.C = (int)(c < kOdeMaxCluster ? c : kOdeMaxCluster);
+    ode_shape(d, &g.T, &g.C);
   } else {
     g.kind = 0;
     g.T = threads;
@@ -1061,6 +1078,11 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
   // profiles, since the autotuner's timings are not representative under a profiler)
   int threads = b->tuned_threads, ppt = b->tuned_ppt, spread = b->tuned_spread;
   if (!threads) pinned_shape(&threads, &ppt, &spread);
+  if (!threads && all_ode) {  // the shape of a fit's CTAs is its own (ode_shape)
+    threads = 256;
+    ppt = 1;
+    spread = 8;
+  }
   if (!threads) {
     const std::string key = shape_key(b);
     {
@@ -1081,10 +1103,8 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
       const int cand_s[2] = {8, 2};
       float best_ms = 1e30f;
       for (int cs : cand_s) {
-        if (cs != 8 && all_ode) continue;  // ODE fits take one particle per thread
         for (int ct : cand_t) {
           for (int cp : cand_p) {
-            if (cp == 2 && all_ode) continue;  // ODE swarms ignore PPT
             if ((rc = run_groups(b, ct, cp, cs, nullptr, nullptr))) return rc;
             PPS_CUDA(cudaEventSynchronize(b->ev1));
             float ms = 0.0f;

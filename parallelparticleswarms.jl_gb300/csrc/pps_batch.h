@@ -63,7 +63,7 @@ void batch_plan(const std::vector<BatchSwarm>& descs, int threads, int ppt, std:
                 std::vector<LaunchGroup>* groups, int spread = 8);
 // a batch of ODE fits alone, its units of work placed on the SMs by cost
 // (pps_ode_teams.cu): every fit's whole run in one cooperative launch.  *taken
-// false: nothing was launched (the device cannot hold the grid); else
+// false: nothing was launched (clusters are faster for these fits, or the device cannot hold the grid); else
 // *error_word is a device word, nonzero after the run if a wait gave up.
 struct OdeTeams;
 OdeTeams* ode_teams_create();

@@ -27,6 +27,7 @@
 // result equals its solve alone, bit for bit (Philox by particle, the argmin
 // over the whole fit).
 #include <algorithm>
+#include <cmath>
 #include <functional>
 #include <new>
 #include <queue>
@@ -256,6 +257,41 @@ static double phase_cost(const BatchSwarm& d) {
 // (700 fits, 30 iterations: 78 ms against 83).
 constexpr int kOdeScalarUnits = 3;
 
+// Whether the units beat one CTA or cluster per fit (k_batch_ode) for this batch,
+// by estimates of both in us.  A phase of a unit costs 2.3 us of its SM beside its
+// steps (state through L2, fence, counters, the next phase's gather) and at least
+// 8 from end to end; a trip of a CTA costs 1.0 and 1.2, a cluster's barriers
+// 3.5.  So short solves and fits that one CTA holds are better off with the CTA,
+// long and large ones with the units, which also fill the SMs evenly.  Measured,
+// ms a batch of 50 iterations, clusters / units: 1 fit of 128 particles and 10 steps
+// 0.16 / 0.42, 400 steps 1.27 / 1.40; 64 of 1024 and 60 steps 0.62 / 0.86, 400
+// steps 2.51 / 2.30; 600 of 4096 and 10 steps 4.4 / 8.5, 60 steps 11.6 / 13.2; 200 of
+// 4096 and 150 steps 9.3 / 8.5; 16 of 16384 and 10 steps 1.44 / 1.09; 1 of 65536 and
+// 400 steps 43 / 2.6.  Over 219 such batches the estimates' choice is within 5 %
+// of the better form in all but a few, and those within 16 %.
+static bool units_pay(const std::vector<BatchSwarm>& descs, int64_t total1, int64_t total2, bool pack, int sm_count) {
+  double chain_u = 0.0, load_u = 0.0, chain_c = 0.0, load_c = 0.0, most = 0.0, ctas = 0.0;
+  for (const auto& d : descs) {
+    const LaunchGroup g = batch_group_of(d, 256, 1);
+    const double steps = ode_cfg(d.op, d.ndata).nsteps, phases = d.maxiters + 1.0, q = g.T / 128.0;
+    const double units = (double)((d.n + kTeam * (pack ? 2 : 1) - 1) / (kTeam * (pack ? 2 : 1)));
+    const double trips = (double)((d.n + 2 * (int64_t)g.T * g.C - 1) / (2 * (int64_t)g.T * g.C));
+    most = std::max(most, phases);
+    chain_u = std::max(chain_u, phases * (pack ? steps * 0.0575 + 9.0 : steps * 0.05));
+    load_u += phases * units * (pack ? steps * 0.04 + 2.3 : steps * 0.03);
+    chain_c = std::max(chain_c, phases * (trips * (steps * std::max(0.0575, 0.052 * q) + 0.6 + 0.6 * q) +
+                                          (g.C > 1 ? 3.5 : 0.0)));
+    load_c += phases * g.C * q * trips * (steps * 0.052 + 1.0);
+    ctas += g.C * q;
+  }
+  // whole units and CTAs per SM
+  const double sm = sm_count, per_u = (double)(pack ? total2 : total1) / sm, per_c = ctas / sm;
+  const double u = pack ? std::max(chain_u, load_u / sm + 3.0 * most)
+                        : std::max(chain_u, load_u / sm * std::ceil(per_u) / per_u) + most * (8.0 + per_u);
+  const double c = std::max(chain_c, load_c / sm * (per_c > 1.0 ? std::ceil(per_c) / per_c : 1.0));
+  return u < c;
+}
+
 struct OdeTeams {
   void* mem = nullptr;
   size_t cap = 0;
@@ -280,7 +316,7 @@ int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSw
   }
   const bool pack = total1 > (int64_t)kOdeScalarUnits * sm_count;
   const int64_t total = pack ? total2 : total1;
-  if (total > (1 << 22)) return PPS_OK;
+  if (total > (1 << 22) || !units_pay(descs, total1, total2, pack, sm_count)) return PPS_OK;
   const int width = kTeam * (pack ? 2 : 1);
   int teams = kMaxTeams;
   while (teams > 1 && sizeof(float) * (size_t)data_floats * teams > (200u << 10)) --teams;
