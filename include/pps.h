@@ -213,12 +213,18 @@ PPS_API int pps_batch_destroy(pps_batch* b);
 /* queue one swarm; *slot identifies it in the results */
 PPS_API int pps_batch_add(pps_batch* b, const pps_problem* prob, int64_t n, uint64_t seed, int32_t maxiters,
                           float w, float wdamp, float c1, float c2, int32_t* slot);
-/* solve every queued swarm in one launch (longest work first); the block
- * shape comes from the autotuner unless pps_batch_set_shape fixed it */
+/* solve every queued swarm together (longest work first).  ODE fits alone and
+ * closed-form swarms alone have forms with nothing to tune; in other batches
+ * the closed forms' block shape comes from the autotuner.  A shape fixed by
+ * pps_batch_set_shape keeps closed forms in the kernel that has it; ODE fits have
+ * shapes of their own */
 PPS_API int pps_batch_run(pps_batch* b, float* device_ms);
 /* threads in {128, 256, 512}, ppt (particles per thread) in {1, 2};
  * (0, 0) returns to autotuning */
 PPS_API int pps_batch_set_shape(pps_batch* b, int32_t threads, int32_t ppt);
+/* threads: the largest block of the last run, ppt: the particles of one of its
+ * threads; device_bytes: what the queued swarms' state, inputs and results take,
+ * with the tables of the last run */
 PPS_API int pps_batch_info(pps_batch* b, int32_t* nswarms, int32_t* threads, int32_t* ppt,
                            uint64_t* device_bytes);
 PPS_API int pps_batch_result(pps_batch* b, int32_t slot, float* u, float* cost, int64_t* idx);

@@ -199,7 +199,7 @@ size_t swarm_device_bytes(const pps_problem* prob, int64_t n) { return swarm_lay
 static int swarm_setup(pps_swarm* s, const pps_problem* prob, int64_t n, uint64_t seed, uint32_t flags, char* b,
                        const SwarmLayout& L, size_t extra = 0) {
   const int D = prob->dim;
-  s->bytes = L.bytes;
+  s->bytes = L.bytes + extra;
   s->dv.X = reinterpret_cast<float*>(b + L.oX);
   s->dv.V = reinterpret_cast<float*>(b + L.oV);
   s->dv.P = reinterpret_cast<float*>(b + L.oP);

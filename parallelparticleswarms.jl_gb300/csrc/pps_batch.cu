@@ -516,24 +516,32 @@ namespace pps {
 
 static size_t a256(size_t v) { return (v + 255) / 256 * 256; }
 
+size_t batch_state_bytes(int D, int64_t ld) {
+  return a256(sizeof(float) * (size_t)D * ld) * 3 + a256(sizeof(float) * ld) * 2;
+}
+
 size_t batch_swarm_bytes(int D, int64_t ld, int64_t ndata) {
-  return a256(sizeof(float) * (size_t)D * ld) * 3 + a256(sizeof(float) * ld) * 2 + a256(sizeof(float) * D) * 4 +
-         256 + a256(sizeof(float) * (size_t)ndata);
+  return batch_state_bytes(D, ld) + a256(sizeof(float) * D) * 4 + 256 + a256(sizeof(float) * (size_t)ndata);
+}
+
+void batch_carve_state(BatchSwarm& d, char* base) {
+  const size_t vec = a256(sizeof(float) * (size_t)d.dim * d.ld), one = a256(sizeof(float) * d.ld);
+  d.X = reinterpret_cast<float*>(base);
+  d.V = reinterpret_cast<float*>(base + vec);
+  d.P = reinterpret_cast<float*>(base + 2 * vec);
+  d.pcost = reinterpret_cast<float*>(base + 3 * vec);
+  d.cost = reinterpret_cast<float*>(base + 3 * vec + one);
 }
 
 void batch_carve(BatchSwarm& d, char* base) {
   const int D = d.dim;
-  size_t off = 0;
+  batch_carve_state(d, base);
+  size_t off = batch_state_bytes(D, d.ld);
   auto take = [&](size_t bytes) {
     char* p = base + off;
     off += a256(bytes);
     return p;
   };
-  d.X = reinterpret_cast<float*>(take(sizeof(float) * (size_t)D * d.ld));
-  d.V = reinterpret_cast<float*>(take(sizeof(float) * (size_t)D * d.ld));
-  d.P = reinterpret_cast<float*>(take(sizeof(float) * (size_t)D * d.ld));
-  d.pcost = reinterpret_cast<float*>(take(sizeof(float) * d.ld));
-  d.cost = reinterpret_cast<float*>(take(sizeof(float) * d.ld));
   d.lb = reinterpret_cast<float*>(take(sizeof(float) * D));
   d.ub = reinterpret_cast<float*>(take(sizeof(float) * D));
   d.u0 = reinterpret_cast<float*>(take(sizeof(float) * D));
@@ -813,6 +821,7 @@ struct pps_batch {
   bool ran = false;
   float* io = nullptr;  // device: every swarm's g and result words, then every swarm's inputs
   size_t io_cap = 0;    // floats
+  size_t io_floats = 0;  // what the queued swarms need of it
   std::vector<size_t> out_at;    // per swarm: its outputs' place in io
   size_t out_floats = 0;
   std::vector<float> outputs;    // the last run's outputs
@@ -848,11 +857,9 @@ int prepare(pps_batch* b) {
   // copy, and its outputs (g, then the result words) in one read by one copy
   // after the run: a copy per swarm and array took 4 ms of a run of 256 swarms,
   // reading the results one by one 5 ms
-  size_t nin = 0, nout = 0;
-  for (size_t k = 0; k < ns; ++k) {
-    nin += b->host[k].size();
-    nout += (size_t)b->descs[k].dim + kResultWords;
-  }
+  size_t nout = 0;
+  for (size_t k = 0; k < ns; ++k) nout += (size_t)b->descs[k].dim + kResultWords;
+  const size_t nin = b->io_floats - nout;
   if (b->io_cap < nin + nout) {
     if (b->io) cudaFree(b->io);
     b->io = nullptr;
@@ -869,7 +876,7 @@ int prepare(pps_batch* b) {
   for (size_t k = 0; k < ns; ++k) {
     BatchSwarm& d = b->descs[k];
     const int D = d.dim;
-    batch_carve(d, base + b->offsets[k]);
+    batch_carve_state(d, base + b->offsets[k]);
     d.mail = nullptr;
     d.done = nullptr;
     d.g = b->io + out;
@@ -1026,7 +1033,8 @@ int pps_batch_add(pps_batch* b, const pps_problem* prob, int64_t n, uint64_t see
   const int rc = batch_describe(prob, n, seed, maxiters, w, wdamp, c1, c2, &d, &h);
   if (rc) return rc;
   b->offsets.push_back(b->arena_bytes);
-  b->arena_bytes += batch_swarm_bytes(d.dim, d.ld, d.ndata);
+  b->arena_bytes += batch_state_bytes(d.dim, d.ld);
+  b->io_floats += h.size() + (size_t)d.dim + kResultWords;
   b->descs.push_back(d);
   b->host.push_back(std::move(h));
   b->ran = false;
@@ -1055,11 +1063,13 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
     if (none_ode && !b->resident && !(b->resident = batch_resident_create()))
       return set_error(PPS_ENOMEM, "host allocation failed");
     bool taken = false;
+    int shape_threads = 0, shape_ppt = 1;
     unsigned int *word = nullptr, timed_out = 0;
     PPS_CUDA(cudaEventRecord(b->ev0, b->stream));
-    rc = all_ode ? ode_teams_launch(b->teams, b->stream, b->descs, b->ddescs, b->sm_count, &taken, &word)
+    rc = all_ode ? ode_teams_launch(b->teams, b->stream, b->descs, b->ddescs, b->sm_count, &taken, &word,
+                                    &shape_threads, &shape_ppt)
                  : batch_resident_launch(b->resident, b->stream, b->descs, b->host, b->ddescs, b->sm_count, &taken,
-                                         &word);
+                                         &word, &shape_threads);
     if (rc) return rc;
     if (taken) {
       PPS_CUDA(cudaEventRecord(b->ev1, b->stream));
@@ -1067,8 +1077,8 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
       if ((rc = read_outputs(b))) return rc;
       if (device_ms) PPS_CUDA(cudaEventElapsedTime(device_ms, b->ev0, b->ev1));
       if (timed_out) return set_error(PPS_ETIMEOUT, "the batch timed out waiting for a swarm's iteration");
-      b->last_threads = all_ode ? 128 : 512;
-      b->last_ppt = 1;
+      b->last_threads = shape_threads;
+      b->last_ppt = shape_ppt;
       b->ran = true;
       return PPS_OK;
     }
@@ -1129,6 +1139,11 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
   if (device_ms) PPS_CUDA(cudaEventElapsedTime(device_ms, b->ev0, b->ev1));
   b->last_threads = threads;
   b->last_ppt = ppt;
+  if (all_ode) {
+    b->last_threads = 0;
+    for (const auto& d : b->descs) b->last_threads = std::max(b->last_threads, batch_group_of(d, threads, ppt).T);
+    b->last_ppt = 2;
+  }
   b->last_spread = spread;
   b->ran = true;
   return PPS_OK;
@@ -1154,7 +1169,9 @@ int pps_batch_info(pps_batch* b, int32_t* nswarms, int32_t* threads, int32_t* pp
   if (nswarms) *nswarms = (int32_t)b->descs.size();
   if (threads) *threads = b->last_threads;
   if (ppt) *ppt = b->last_ppt;
-  if (device_bytes) *device_bytes = b->arena_bytes;
+  if (device_bytes)
+    *device_bytes = b->arena_bytes + sizeof(float) * b->io_floats + (sizeof(BatchSwarm) + sizeof(int)) * b->descs.size() +
+                    ode_teams_bytes(b->teams) + batch_resident_bytes(b->resident);
   return PPS_OK;
 }
 

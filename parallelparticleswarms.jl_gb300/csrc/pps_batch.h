@@ -45,6 +45,9 @@ struct LaunchGroup {
 size_t batch_swarm_bytes(int dim, int64_t ld, int64_t ndata);
 // carve a swarm's regions from `base` (256-byte aligned)
 void batch_carve(BatchSwarm& d, char* base);
+// the same for the state alone (X, V, P, pcost, cost), where the rest lies elsewhere
+size_t batch_state_bytes(int dim, int64_t ld);
+void batch_carve_state(BatchSwarm& d, char* base);
 double batch_work_estimate(const BatchSwarm& d);
 // validate a problem for batching and fill a descriptor (no device pointers);
 // host_inputs receives lb | ub | u0 | data
@@ -54,8 +57,8 @@ size_t batch_smem_bytes(int maxdim, int data_floats, int64_t maxchunk);
 // the (kind, T, C) a swarm is launched with: separable swarms use the
 // batch's block size and about `spread` particles per thread per iteration
 // (8 by default; fewer split a swarm over more CTAs), ODE fits two particles
-// per thread (their RK4 losses packed; up to 1024 threads per CTA), both
-// split over up to 16 CTAs
+// per thread (their RK4 losses packed) in CTAs sized by their steps, both split
+// over up to 16 CTAs
 LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread = 8);
 // group swarms by (kind, T, C); order lists descriptor indices group by
 // group, longest estimated work first inside each group
@@ -63,22 +66,26 @@ void batch_plan(const std::vector<BatchSwarm>& descs, int threads, int ppt, std:
                 std::vector<LaunchGroup>* groups, int spread = 8);
 // a batch of ODE fits alone, its units of work placed on the SMs by cost
 // (pps_ode_teams.cu): every fit's whole run in one cooperative launch.  *taken
-// false: nothing was launched (clusters are faster for these fits, or the device cannot hold the grid); else
-// *error_word is a device word, nonzero after the run if a wait gave up.
+// false: nothing was launched (one CTA or cluster per fit is faster for these,
+// or the device cannot hold the grid); else
+// *error_word is a device word, nonzero after the run if a wait gave up, and
+// *threads, *ppt are its largest block and the particles of a thread.
 struct OdeTeams;
 OdeTeams* ode_teams_create();
 void ode_teams_destroy(OdeTeams* t);
+size_t ode_teams_bytes(const OdeTeams* t);  // device bytes it keeps
 int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSwarm>& descs, const BatchSwarm* ddescs,
-                     int sm_count, bool* taken, unsigned int** error_word);
+                     int sm_count, bool* taken, unsigned int** error_word, int* threads, int* ppt);
 // a batch of closed-form swarms alone, resident in shared memory wave by wave
 // (pps_batch_resident.cu); host: per swarm lb | ub | ...  *taken, *error_word
 // as for ode_teams_launch (*taken also false where a swarm does not fit the form).
 struct BatchResident;
 BatchResident* batch_resident_create();
 void batch_resident_destroy(BatchResident* t);
+size_t batch_resident_bytes(const BatchResident* t);
 int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vector<BatchSwarm>& descs,
                           const std::vector<std::vector<float>>& host, const BatchSwarm* ddescs, int sm_count,
-                          bool* taken, unsigned int** error_word);
+                          bool* taken, unsigned int** error_word, int* threads);
 // launch one group: descs[dorder[g.offset + k]], k < g.count, on `stream`
 int batch_launch_group(cudaStream_t stream, const BatchSwarm* ddescs, const int* dorder, const LaunchGroup& g,
                        int ppt);

@@ -148,6 +148,8 @@ void batch_resident_destroy(BatchResident* t) {
   delete t;
 }
 
+size_t batch_resident_bytes(const BatchResident* t) { return t ? t->cap : 0; }
+
 // the blocks' limits with `per` of them on an SM
 constexpr size_t kJobStatic = 6u << 10;  // static shared memory of k_batch_resident, and the driver's 1 kB a block
 static int most_threads(int per) { return kResidentThreads / per; }
@@ -159,7 +161,7 @@ static int64_t coords_of(const BatchSwarm& d) { return d.n * (int64_t)((d.dim + 
 
 int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vector<BatchSwarm>& descs,
                           const std::vector<std::vector<float>>& host, const BatchSwarm* ddescs, int sm_count,
-                          bool* taken, unsigned int** error_word) {
+                          bool* taken, unsigned int** error_word, int* threads) {
   *taken = false;
   const int ns = (int)descs.size();
   // blocks per SM: one of 512 threads, or more and smaller ones while the
@@ -235,7 +237,7 @@ int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vect
       most.push({coords_of(descs[w[e]]) / blocks[e], e});
     }
     size_t smem = 0;
-    int threads = 32;
+    int block = 32;
     for (size_t e = 0; e < w.size(); ++e) {
       const BatchSwarm& d = descs[w[e]];
       ResidentPlan p;
@@ -274,11 +276,11 @@ int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vect
       for (int r = 0; r < p.blocks; ++r) table.push_back(make_int2((int)jobs.size(), r));
       jobs.push_back(j);
       smem = std::max(smem, p.smem);
-      threads = std::max(threads, p.threads);
+      block = std::max(block, p.threads);
     }
     wave_at.push_back((int)table.size());
     wave_smem.push_back(smem);
-    wave_threads.push_back(threads);
+    wave_threads.push_back(block);
   }
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   const size_t bxch = up(sizeof(unsigned long long) * xch_words + sizeof(unsigned int));
@@ -330,6 +332,8 @@ int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vect
     if (e != cudaSuccess) return cuda_error(e, "cudaLaunchKernelEx(k_batch_resident)");
   }
   *error_word = status;
+  *threads = kBatchInitThreads;  // the sampling's block, where no swarm has an iteration to run
+  if (!jobs.empty()) *threads = *std::max_element(wave_threads.begin(), wave_threads.end());
   *taken = true;
   return PPS_OK;
 }

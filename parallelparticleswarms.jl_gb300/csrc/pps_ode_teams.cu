@@ -303,8 +303,10 @@ void ode_teams_destroy(OdeTeams* t) {
   delete t;
 }
 
+size_t ode_teams_bytes(const OdeTeams* t) { return t ? t->cap : 0; }
+
 int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSwarm>& descs, const BatchSwarm* ddescs,
-                     int sm_count, bool* taken, unsigned int** error_word) {
+                     int sm_count, bool* taken, unsigned int** error_word, int* threads, int* ppt) {
   *taken = false;
   const int nf = (int)descs.size();
   int64_t total1 = 0, total2 = 0;
@@ -396,6 +398,8 @@ int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSw
   }
   if (e != cudaSuccess) return cuda_error(e, "cudaLaunchKernelEx(k_ode_teams)");
   *error_word = &ctl[nf].phase;
+  *threads = teams * kTeam;
+  *ppt = pack ? 2 : 1;
   *taken = true;
   return PPS_OK;
 }
