@@ -742,6 +742,8 @@ void batch_plan(const std::vector<BatchSwarm>& descs, int threads, int ppt, std:
   }
 }
 
+constexpr size_t kBatchSmem = 200u << 10;  // dynamic shared memory of a CTA
+
 // Launch a group with clusters of g.C CTAs, or of a smaller size when the
 // device cannot co-schedule that many with this block shape.  How a swarm is
 // split over CTAs does not change its result (draws are keyed by particle,
@@ -749,12 +751,12 @@ void batch_plan(const std::vector<BatchSwarm>& descs, int threads, int ppt, std:
 template <typename Kernel>
 static int launch_clustered(Kernel kernel, cudaStream_t stream, const BatchSwarm* ddescs, const int* dorder,
                             const LaunchGroup& g, int width) {
-  cudaError_t e = cudaSuccess;
+  // the limit is the process's: a constant, so no other thread lowers it before the launch
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmem);
+  if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute");
   for (int C = g.C; C >= 1; C = (C > 8 ? 8 : C / 2)) {
     const size_t smem = batch_smem_bytes(g.maxdim, g.data_floats, chunk_of(g.maxn, C, width));
-    if (smem > 200 * 1024) continue;
-    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-      return cuda_error(e, "cudaFuncSetAttribute");
+    if (smem > kBatchSmem) continue;
     if (C > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
       cudaGetLastError();
       continue;

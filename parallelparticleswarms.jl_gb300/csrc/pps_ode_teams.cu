@@ -41,6 +41,7 @@ namespace pps {
 
 constexpr int kTeam = 128;
 constexpr int kMaxTeams = 8;
+constexpr size_t kOdeTeamSmem = 200u << 10;  // observations of a block's teams
 constexpr unsigned int kOdeTeamLooks = 1u << 30;  // many minutes: phases of very long fits end in seconds
 
 // control words of one fit, zero at launch; the entry behind the last fit holds the run's error word in `phase`
@@ -321,7 +322,7 @@ int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSw
   if (total > (1 << 22) || !units_pay(descs, total1, total2, pack, sm_count)) return PPS_OK;
   const int width = kTeam * (pack ? 2 : 1);
   int teams = kMaxTeams;
-  while (teams > 1 && sizeof(float) * (size_t)data_floats * teams > (200u << 10)) --teams;
+  while (teams > 1 && sizeof(float) * (size_t)data_floats * teams > kOdeTeamSmem) --teams;
   const int blocks = (int)std::min<int64_t>(sm_count, total);
   teams = (int)std::min<int64_t>(teams, (total + blocks - 1) / blocks);
   // longest fits first, each unit onto the least loaded block, within it onto the least loaded team
@@ -378,8 +379,8 @@ int ode_teams_launch(OdeTeams* t, cudaStream_t stream, const std::vector<BatchSw
   PPS_CUDA(cudaMemcpyAsync(doff, offsets.data(), sizeof(int) * offsets.size(), cudaMemcpyHostToDevice, stream));
   const size_t smem = sizeof(float) * (size_t)data_floats * teams;
   auto kernel = pack ? k_ode_teams<true> : k_ode_teams<false>;
-  if (smem > (40u << 10))
-    PPS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the limit is the process's: a constant, so no other thread lowers it before the launch
+  PPS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOdeTeamSmem));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)(teams * kTeam));
