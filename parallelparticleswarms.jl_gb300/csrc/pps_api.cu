@@ -333,6 +333,7 @@ int swarm_create(const pps_problem* prob, int64_t n, uint64_t seed, uint32_t fla
     s->stream = ps.stream;
     s->ev0 = ps.ev0;
     s->ev1 = ps.ev1;
+    s->stream_context = ps.context;
     s->pooled = L.bytes + xch <= kPooledBlock;
     e = s->pooled ? pool_alloc(s->device, &s->block, L.bytes + xch, s->stream) : cudaMalloc(&s->block, L.bytes + xch);
     if (e != cudaSuccess) {
@@ -384,7 +385,7 @@ int pps_swarm_destroy(pps_swarm* s) {
       cudaFree(s->block);
   }
   if (s->local_block) cudaFree(s->local_block);
-  PoolStream ps{s->stream, s->ev0, s->ev1};
+  PoolStream ps{s->stream, s->ev0, s->ev1, s->stream_context};
   pool_stream_put(s->device, &ps);
   free(s->host_lb);
   if (dev >= 0 && dev != s->device) cudaSetDevice(dev);

@@ -29,6 +29,7 @@ struct ObjData {
 struct pps_swarm {
   int device = 0;
   cudaStream_t stream = nullptr;
+  unsigned long long stream_context = 0;  // PoolStream::context of stream, ev0 and ev1
   void* block = nullptr;  // the single device allocation
   bool pooled = false;    // block came from pool_alloc (freed in the stream's order)
   size_t bytes = 0;

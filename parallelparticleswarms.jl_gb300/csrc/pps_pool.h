@@ -20,6 +20,7 @@ constexpr size_t kPoolBytes = (size_t)64 << 20;
 struct PoolStream {
   cudaStream_t stream = nullptr;  // non-blocking
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  unsigned long long context = 0;  // the context it belongs to (0: it is not kept)
 };
 
 // a stream of the current device, idle
