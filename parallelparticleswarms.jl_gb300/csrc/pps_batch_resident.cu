@@ -48,14 +48,14 @@ struct ResidentJob {
   int split;
 };
 
-// Sampling and the first global best, one block per swarm (src/utils.jl:57-84,
-// src/init.jl:102-106).
+// Sampling and the first global best (src/utils.jl:57-84, src/init.jl:102-106) by
+// `share` blocks of one swarm, this one `rank` of them.
 constexpr int kBatchInitThreads = 512;
 template <int OBJ>
-__device__ __forceinline__ unsigned long long init_swarm(const BatchSwarm& sw) {
+__device__ __forceinline__ unsigned long long init_swarm(const BatchSwarm& sw, int rank, int share) {
   const uint32_t k0 = (uint32_t)sw.seed, k1 = (uint32_t)(sw.seed >> 32);
   unsigned long long best = ~0ull;
-  for (int64_t i = threadIdx.x; i < sw.n; i += blockDim.x) {
+  for (int64_t i = (int64_t)rank * blockDim.x + threadIdx.x; i < sw.n; i += (int64_t)share * blockDim.x) {
     Acc<OBJ> acc;
     for (int j = 0; j < sw.dim; j += 4) {
       const Rand4 r = philox4x32_10((uint32_t)i, (uint32_t)(j >> 2), 0u, kTagInit, k0, k1);
@@ -89,24 +89,54 @@ __device__ __forceinline__ unsigned long long init_swarm(const BatchSwarm& sw) {
   return best;
 }
 
-__global__ void __launch_bounds__(kBatchInitThreads) k_batch_init(const BatchSwarm* __restrict__ descs) {
+// one swarm's sampling across blocks, zero at launch
+struct InitCtl {
+  unsigned long long inv_key;  // ~ the lowest argmin key so far
+  unsigned int done;           // blocks finished
+  unsigned int pad;
+};
+
+// Block (r, k) samples its share of swarm k; the last of the swarm's blocks takes
+// the global best.  As many blocks a swarm as fill the GPU (a sampling alone, us
+// with one / with these / by the streaming form's clusters: one swarm of 20,000 x 128-D
+// 714 / 60 / 232, four 980 / 102 / 361).
+__global__ void __launch_bounds__(kBatchInitThreads)
+    k_batch_init(const BatchSwarm* __restrict__ descs, InitCtl* __restrict__ ctls) {
   __shared__ unsigned long long red[kBatchInitThreads / 32];
-  const BatchSwarm sw = descs[blockIdx.x];
+  __shared__ unsigned long long win_s;
+  __shared__ int last_s;
+  const BatchSwarm sw = descs[blockIdx.y];
+  const int most = (int)((sw.n + kBatchInitThreads - 1) / kBatchInitThreads);
+  const int share = most < (int)gridDim.x ? most : (int)gridDim.x, rank = (int)blockIdx.x;
+  if (rank >= share) return;
   unsigned long long best = ~0ull;
   switch (sw.objective) {
-    case kSphere: best = init_swarm<kSphere>(sw); break;
-    case kRosenbrock: best = init_swarm<kRosenbrock>(sw); break;
-    case kRastrigin: best = init_swarm<kRastrigin>(sw); break;
-    default: best = init_swarm<kAckley>(sw); break;
+    case kSphere: best = init_swarm<kSphere>(sw, rank, share); break;
+    case kRosenbrock: best = init_swarm<kRosenbrock>(sw, rank, share); break;
+    case kRastrigin: best = init_swarm<kRastrigin>(sw, rank, share); break;
+    default: best = init_swarm<kAckley>(sw, rank, share); break;
   }
   best = warp_min_key(best);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
-  __syncthreads();  // also orders the block's writes of P and pcost before the reads below
-  best = warp_min_key((threadIdx.x & 31) < kBatchInitThreads / 32 ? red[threadIdx.x & 31] : ~0ull);
-  const int64_t gi = (int64_t)(uint32_t)best;
-  for (int d = threadIdx.x; d < sw.dim; d += blockDim.x) sw.g[d] = sw.P[(int64_t)d * sw.ld + gi];
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = warp_min_key(threadIdx.x < kBatchInitThreads / 32 ? red[threadIdx.x] : ~0ull);
+    if (threadIdx.x == 0) {
+      InitCtl* c = ctls + blockIdx.y;
+      atomicMax(&c->inv_key, ~best);  // inverted, so zeroed memory is "none yet"
+      __threadfence();
+      last_s = atomicAdd(&c->done, 1u) == (unsigned int)(share - 1);
+      __threadfence();
+      if (last_s) win_s = ~atomicMax(&c->inv_key, 0ull);
+    }
+  }
+  __syncthreads();
+  if (!last_s) return;
+  const int64_t gi = (int64_t)(uint32_t)win_s;
+  for (int d = threadIdx.x; d < sw.dim; d += blockDim.x) sw.g[d] = __ldcg(sw.P + (int64_t)d * sw.ld + gi);
   if (threadIdx.x == 0) {
-    sw.result[0] = sw.pcost[gi];
+    sw.result[0] = __ldcg(sw.pcost + gi);
     sw.result[1] = __uint_as_float((uint32_t)gi);
     sw.result[2] = 0.0f;
   }
@@ -283,8 +313,10 @@ int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vect
     wave_threads.push_back(block);
   }
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-  const size_t bxch = up(sizeof(unsigned long long) * xch_words + sizeof(unsigned int));
-  const size_t bjobs = up(sizeof(ResidentJob) * jobs.size()), need = bxch + bjobs + sizeof(int2) * table.size() + 256;
+  // zeroed: the samplings' words, the exchange words, the error word
+  const size_t binit = sizeof(InitCtl) * (size_t)ns;
+  const size_t bzero = up(binit + sizeof(unsigned long long) * xch_words + sizeof(unsigned int));
+  const size_t bjobs = up(sizeof(ResidentJob) * jobs.size()), need = bzero + bjobs + sizeof(int2) * table.size() + 256;
   if (t->cap < need) {
     if (t->mem) cudaFree(t->mem);
     t->mem = nullptr;
@@ -293,22 +325,27 @@ int batch_resident_launch(BatchResident* t, cudaStream_t stream, const std::vect
     t->cap = need;
   }
   char* m = static_cast<char*>(t->mem);
-  unsigned long long* xch = reinterpret_cast<unsigned long long*>(m);
+  unsigned long long* xch = reinterpret_cast<unsigned long long*>(m + binit);
   unsigned int* status = reinterpret_cast<unsigned int*>(xch + xch_words);
   for (size_t k = 0; k < jobs.size(); ++k) {
     jobs[k].a.xch = xch + job_xch[k];
     jobs[k].a.status = status;
   }
-  ResidentJob* djobs = reinterpret_cast<ResidentJob*>(m + bxch);
-  int2* dtable = reinterpret_cast<int2*>(m + bxch + bjobs);
-  PPS_CUDA(cudaMemsetAsync(m, 0, bxch, stream));
+  ResidentJob* djobs = reinterpret_cast<ResidentJob*>(m + bzero);
+  int2* dtable = reinterpret_cast<int2*>(m + bzero + bjobs);
+  PPS_CUDA(cudaMemsetAsync(m, 0, bzero, stream));
   if (!jobs.empty()) {
     PPS_CUDA(cudaMemcpyAsync(djobs, jobs.data(), sizeof(ResidentJob) * jobs.size(), cudaMemcpyHostToDevice, stream));
     PPS_CUDA(cudaMemcpyAsync(dtable, table.data(), sizeof(int2) * table.size(), cudaMemcpyHostToDevice, stream));
     PPS_CUDA(cudaFuncSetAttribute(k_batch_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)most_smem(1)));
   }
-  k_batch_init<<<(unsigned)ns, kBatchInitThreads, 0, stream>>>(ddescs);
+  int64_t longest = 1;
+  for (const auto& d : descs) longest = std::max(longest, d.n);
+  const int64_t fill = std::max(8 * sm_count / ns, 1), most = (longest + kBatchInitThreads - 1) / kBatchInitThreads;
+  // (y: the waves hold far fewer swarms than a grid's 65,535)
+  k_batch_init<<<dim3((unsigned)std::min(fill, most), (unsigned)ns), kBatchInitThreads, 0, stream>>>(
+      ddescs, reinterpret_cast<InitCtl*>(m));
   PPS_CUDA(cudaGetLastError());
   for (size_t v = 0; v < waves.size(); ++v) {
     const int nblocks = wave_at[v + 1] - wave_at[v];

@@ -1,0 +1,35 @@
+"""Which form a call takes: short runs, batches of few iterations and mixed
+batches are no slower than in another form of the same work that the library
+has, and equal it bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(pps, name, D, cons=False):
+    f = pps.REGISTRY[name]
+    rows = pps.quadratic_constraint(D, c=-6.25 * D, b=np.ones(D)) if cons else None
+    return pps.OptimizationProblem(f, np.zeros(D, np.float32), list(f.default_params) or None,
+                                   lb=np.full(D, -5.0, np.float32), ub=np.full(D, 5.0, np.float32), cons=rows)
+
+
+@pytest.mark.parametrize("count,n", [(1, 1), (1, 511), (3, 512), (2, 513), (1, 20000), (4, 20000), (200, 1100), (320, 700)])
+def test_batch_sampling(pps, count, n):
+    def run(shape):
+        with pps.Batch() as b:
+            if shape:
+                b.set_shape(*shape)
+            for k in range(count):
+                b.add(_problem(pps, ("sphere", "rosenbrock", "rastrigin", "ackley")[k % 4], 40), n, maxiters=0, seed=k)
+            b.run()
+            ms = min(b.run() for _ in range(9))
+            return ms, [b.result(k) for k in range(count)], b.state(count - 1)
+    ms, got, state = run(None)
+    fixed, want, ref = run((256, 1))
+    for a, b in zip(got, want):
+        assert np.array_equal(a[0], b[0]) and a[1:] == b[1:]
+    for f in ref:
+        assert np.array_equal(state[f], ref[f])
+    if count <= 4:
+        assert ms <= 1.3 * fixed + 0.02
