@@ -534,16 +534,18 @@ static int run_steps(pps_swarm* s, int32_t maxiters, float c1, float c2, uint32_
   return PPS_OK;
 }
 
-// Runs of one iteration (two of a user objective with many particles) whose
-// dims are few stay stepwise: a cooperative launch, the state in and out and a
-// status read cost more than the step saves.  One iteration, us a call, stepwise /
-// resident: sphere 20000 x 2 29.0 / 32.4, 10^6 x 2 39.7 / 46.0, 300000 x 7 40.3 /
-// 44.1, 200000 x 10 38.1 / 43.7, but 65536 x 10 36.1 / 31.6, 100003 x 20 49.1 / 43.9;
-// two: sphere 10^6 x 2 57.9 / 56.9, a user objective there 60.9 / 68.6.
-static bool few_steps(const pps_swarm* s, int32_t maxiters) {
-  if (maxiters > 2) return false;
-  const bool few_dims = s->dv.dim <= 8 || (s->dv.dim <= 16 && s->dv.n > 100000);
-  return few_dims && (maxiters == 1 || (is_user(s->objective) && s->dv.n > 300000));
+// Runs of one or two iterations that stay stepwise: a cooperative launch, the
+// state in and out and a status read cost more than the step saves.  Over 638 shapes of
+// six objectives, resident / stepwise, one iteration: 1000 x 2 1.15, 20000 x 7
+// 0.95-1.05, 300 x 9 1.07, 50000 x 14 0.95-1.06, x 20 0.90-1.07, x 32 0.88-0.98,
+// 100000 x 10 0.91-1.17, x 17 1.01-1.08, 140000 x 10 0.94-1.27; two: 140000 x 10
+// 0.85-0.95, 200000 x 2 0.88-1.10, 500000 x 3 0.94-1.09; three: at most 1.05.
+static bool few_steps(const pps_swarm* s, int32_t maxiters, const ResidentPlan& p) {
+  const int64_t n = s->dv.n;
+  const int D = s->dv.dim;
+  if (maxiters == 1)
+    return n > 60000 || (n > 40000 && D > 16 && D <= 28) || D <= (n <= 1000 ? 10 : 8) || (D > 256 && !p.split);
+  return maxiters == 2 && n > 180000;
 }
 
 // whether a run of this swarm keeps its state on chip (pps_resident.cu):
@@ -553,7 +555,7 @@ static bool resident_applies(const pps_swarm* s, int32_t maxiters, float c1, flo
   if (s->shard || !s->owns_memory || !pair_form(s, c1, c2)) return false;
   if (sync_bulk_requested()) return false;
   if (!resident_plan(s->objective, s->dv.dim, s->dv.n, s->dv.ncons, s->sm_count, plan)) return false;
-  return plan->blocks == 1 || (s->xch_dev && !few_steps(s, maxiters));
+  return plan->blocks == 1 || (s->xch_dev && !few_steps(s, maxiters, *plan));
 }
 
 static int sync_like_run(pps_swarm* s, int32_t maxiters, float w, float wdamp, float c1, float c2,

@@ -6,12 +6,23 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+GENERAL = dict(c1=1e-35, c2=1e-35)  # coefficients that only the general arithmetic takes
+
 
 def _problem(pps, name, D, cons=False):
     f = pps.REGISTRY[name]
     rows = pps.quadratic_constraint(D, c=-6.25 * D, b=np.ones(D)) if cons else None
     return pps.OptimizationProblem(f, np.zeros(D, np.float32), list(f.default_params) or None,
                                    lb=np.full(D, -5.0, np.float32), ub=np.full(D, 5.0, np.float32), cons=rows)
+
+
+@pytest.mark.parametrize("name,D,n,cons", [("sphere", 10, 140000, False), ("sphere", 10, 100000, True)])
+def test_one_synchronous_iteration(pps, name, D, n, cons):
+    with pps.Swarm(_problem(pps, name, D, cons), n, seed=1) as sw:
+        sw.init()
+        short = min(sw.sync_run(1) for _ in range(40))
+        general = min(sw.sync_run(1, **GENERAL) for _ in range(40))
+    assert short <= 1.12 * general
 
 
 @pytest.mark.parametrize("count,n", [(1, 1), (1, 511), (3, 512), (2, 513), (1, 20000), (4, 20000), (200, 1100), (320, 700)])
