@@ -51,8 +51,8 @@ __device__ __forceinline__ void async_publish(const SwarmDev& s, unsigned long l
 // instructions per dim and warp, a branch per pair, 58 % of the issue slots
 // used), this form unpacked 4.68 ms, packed 4.51 ms (50 instructions, 62 %).
 // Two blocks of 128 registers an SM; asking for one or three: 4.89 / 4.73 ms.
-template <int OBJ, int S>
-__global__ void __launch_bounds__(kAsyncThreads, 2) k_async_slice(SwarmDev s, ObjParams op, PhiloxKeys keys, int iters,
+template <int OBJ, int S, int BLOCKS>
+__global__ void __launch_bounds__(kAsyncThreads, BLOCKS) k_async_slice(SwarmDev s, ObjParams op, PhiloxKeys keys, int iters,
                                                                 float c1s, float c2s, int lanes, float one) {
   extern __shared__ __align__(16) float sm[];
   const int D = s.dim;
@@ -332,9 +332,30 @@ static int launch_async_obj(pps_swarm* s, int iters, float c1, float c2, int lan
   const PhiloxKeys keys = philox_round_keys(s->seed);
   const size_t smem = 3 * sizeof(float) * (size_t)lanes * slice;
   const float c1s = c1 * 0x1p-24f, c2s = c2 * 0x1p-24f;
-#define L_SLICE(S) \
-  case S: k_async_slice<OBJ, S><<<(unsigned)blocks, kAsyncThreads, smem, s->stream>>>(s->dv, s->op, keys, iters, c1s, c2s, lanes, 1.0f); break
-  if (slice <= 16 && pair_form(s, c1, c2)) {
+  // Blocks an SM (registers a thread): two, and three or four for slices of 4 to 8
+  // where the grid has more than one round of two and the run is short, or more
+  // than two rounds.  There the loads of the state count, which more warps
+  // overlap: 10^6 x 8-D sphere, us a run of 1 / 5 iterations, two blocks 115 / 156,
+  // three 90 / 122, k_async 91 / 132.  Few blocks gain nothing from the cap on registers:
+  // 10,000 x 8-D, 100 iterations, 72.5 with two, 80.8 with three.  Up to three
+  // iterations take k_async where that is so and where a slice has at most four dims: 10^6 x
+  // 5-D, one iteration 62, three blocks 67; 10,000 x 3-D 24 and 26.
+  const int64_t round = 2 * (int64_t)s->sm_count;
+  const bool many = blocks > round && (iters <= 10 || blocks > 2 * round);
+#define L_SLICE_B(S, B) \
+  k_async_slice<OBJ, S, B><<<(unsigned)blocks, kAsyncThreads, smem, s->stream>>>(s->dv, s->op, keys, iters, c1s, c2s, lanes, 1.0f)
+#define L_SLICE(S)                                      \
+  case S:                                               \
+    if constexpr (S >= 4 && S <= 8) {                   \
+      if (many) {                                       \
+        L_SLICE_B(S, S == 4 ? 4 : 3);                   \
+        break;                                          \
+      }                                                 \
+    }                                                   \
+    L_SLICE_B(S, 2);                                    \
+    break
+  const bool brief = iters <= 3 && (slice <= 4 || (slice <= 8 && blocks > 2 * round));
+  if (slice <= 16 && !brief && pair_form(s, c1, c2)) {
     if constexpr (OBJ >= kBeale) {  // closed forms of at most two dims
       switch (slice) { L_SLICE(2); }
     } else {
@@ -366,6 +387,7 @@ static int launch_async_obj(pps_swarm* s, int iters, float c1, float c2, int lan
     }
   }
 #undef L_SLICE
+#undef L_SLICE_B
 #undef L_GENERAL
   PPS_CUDA(cudaGetLastError());
   return PPS_OK;

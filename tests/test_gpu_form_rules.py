@@ -4,6 +4,8 @@ has, and equal it bit for bit."""
 import numpy as np
 import pytest
 
+from test_gpu_sync_parity import assert_state_equal
+
 pytestmark = pytest.mark.gpu
 
 GENERAL = dict(c1=1e-35, c2=1e-35)  # coefficients that only the general arithmetic takes
@@ -23,6 +25,28 @@ def test_one_synchronous_iteration(pps, name, D, n, cons):
         short = min(sw.sync_run(1) for _ in range(40))
         general = min(sw.sync_run(1, **GENERAL) for _ in range(40))
     assert short <= 1.12 * general
+
+
+@pytest.mark.parametrize("D", [3, 5, 8])
+def test_one_asynchronous_iteration(pps, D):
+    with pps.Swarm(_problem(pps, "sphere", D), 1000000, seed=1) as sw:
+        sw.init()
+        short = min(sw.async_run(1) for _ in range(40))
+        general = min(sw.async_run(1, **GENERAL) for _ in range(40))
+    assert short <= 1.12 * general
+
+
+@pytest.mark.parametrize("n", [1000, 160001])  # both sides of the grid's second round
+@pytest.mark.parametrize("D", [4, 5, 8])
+def test_asynchronous_runs_in_pieces(pps, orc, n, D):
+    prob = _problem(pps, "rastrigin", D)
+    ref = orc.OracleSwarm(orc.OracleProblem(2, D, prob.lb, prob.ub, params=[10.0]), n, 5).init()
+    with pps.Swarm(prob, n, seed=5) as sw:
+        sw.init()
+        for k in (1, 3, 4, 11):
+            sw.async_run(k)
+            ref.async_run(k)
+        assert_state_equal(sw, ref, "after the pieces")
 
 
 @pytest.mark.parametrize("count,n", [(1, 1), (1, 511), (3, 512), (2, 513), (1, 20000), (4, 20000), (200, 1100), (320, 700)])
