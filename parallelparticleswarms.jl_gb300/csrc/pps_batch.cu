@@ -665,27 +665,47 @@ static int ode_threads() {  // 0: not given
 // particles and 10 steps 2.2 / 4.8, 60 steps 7.0 / 7.5, 150 steps 15.9 / 12.7; of
 // 1024 and 10 steps 3.7 / 4.6, 30 steps 7.7 / 5.7; of 4096 and 30 steps 11.0 /
 // 11.6, 60 steps 16.8 / 15.0; 64 of 16384 and 10 steps 43 / 52, 30 steps 73 / 82.
-static void ode_shape(const BatchSwarm& d, int* threads, int* cluster) {
-  const int steps = ode_cfg(d.op, d.ndata).nsteps, given = ode_threads();
-  const bool brief = steps < (d.n <= 512 ? 64 : d.n <= 2048 ? 24 : 32);
+static bool brief_fit(const BatchSwarm& d) {
+  return ode_cfg(d.op, d.ndata).nsteps < (d.n <= 512 ? 64 : d.n <= 2048 ? 24 : 32);
+}
+// Long fits of many particles keep all their threads busy in whatever CTAs, so
+// those should spread evenly over the SMs: 256 threads and eight CTAs a fit, or 512
+// and four, whichever still gives each CTA an SM of its own; with more fits
+// the SMs are full and small CTAs balance best.  Ms, ten iterations beside four
+// small swarms, 128 x 8 / 256 x 8 / 512 x 4: 8 LV fits of 8192 particles and 1000
+// steps 2.7 / 1.9 / 3.8, 16 of 16384 8.3 / 7.1 / 7.5, 24 of 8192 5.0 / 5.0 / 3.6, 24 FHN 6.2 /
+// 6.9 / 4.9, 38 FHN and 400 steps 3.5 / 3.6 / 4.0.
+constexpr int64_t kLargeFit = 4096;
+static bool large_fit(const BatchSwarm& d) { return is_ode(d.objective) && d.n >= kLargeFit && !brief_fit(d); }
+// `large`: how many such fits run together (0: not known)
+static void ode_shape(const BatchSwarm& d, int large, int sm_count, int* threads, int* cluster) {
+  const int given = ode_threads();
+  bool wide = brief_fit(d) || given;
   int T = 128;
-  if (brief || given) {
+  if (large > 0 && large_fit(d)) {
+    if (8 * large <= sm_count)
+      T = 256;
+    else
+      wide = wide || 4 * large <= sm_count - sm_count / 10;
+  }
+  if (wide) {
     const int64_t half = (d.n + 1) / 2;
     const int most = given ? given : 512;
+    T = 128;
     while (T < half && 2 * T <= most) T *= 2;
   }
   const int64_t c = (d.n + 2 * (int64_t)T - 1) / (2 * (int64_t)T);
-  const int cmax = max_cluster(brief || given ? 4 : 8);
+  const int cmax = max_cluster(wide ? 4 : 8);
   *threads = T;
   *cluster = (int)(c < cmax ? c : cmax);
 }
 
-LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread) {
+LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread, int large, int sm_count) {
   LaunchGroup g{};
   const int cmax = max_cluster(4);
   if (is_ode(d.objective)) {
     g.kind = 1;
-    ode_shape(d, &g.T, &g.C);
+    ode_shape(d, large, sm_count, &g.T, &g.C);
   } else {
     g.kind = 0;
     g.T = threads;
@@ -711,11 +731,13 @@ LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread
 static int64_t chunk_of(int64_t n, int C, int width) { return cta_chunk(n, C, width); }
 
 void batch_plan(const std::vector<BatchSwarm>& descs, int threads, int ppt, std::vector<int>* order,
-                std::vector<LaunchGroup>* groups, int spread) {
+                std::vector<LaunchGroup>* groups, int spread, int sm_count) {
   const int ns = (int)descs.size();
+  int large = 0;
+  for (const auto& d : descs) large += large_fit(d);
   std::map<std::tuple<int, int, int>, std::vector<int>> by;
   for (int k = 0; k < ns; ++k) {
-    const LaunchGroup g = batch_group_of(descs[k], threads, ppt, spread);
+    const LaunchGroup g = batch_group_of(descs[k], threads, ppt, spread, large, sm_count);
     by[std::make_tuple(-g.C, g.kind, g.T)].push_back(k);  // larger clusters first
   }
   order->clear();
@@ -909,7 +931,7 @@ int read_outputs(pps_batch* b) {
 int run_groups(pps_batch* b, int threads, int ppt, int spread, int* ngroups, int* maxc) {
   std::vector<int> order;
   std::vector<LaunchGroup> groups;
-  batch_plan(b->descs, threads, ppt, &order, &groups, spread);
+  batch_plan(b->descs, threads, ppt, &order, &groups, spread, b->sm_count);
   PPS_CUDA(cudaMemcpyAsync(b->dorder, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, b->stream));
   PPS_CUDA(cudaEventRecord(b->ev0, b->stream));
   int rc = PPS_OK;

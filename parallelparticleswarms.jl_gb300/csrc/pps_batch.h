@@ -57,13 +57,15 @@ size_t batch_smem_bytes(int maxdim, int data_floats, int64_t maxchunk);
 // the (kind, T, C) a swarm is launched with: separable swarms use the
 // batch's block size and about `spread` particles per thread per iteration
 // (8 by default; fewer split a swarm over more CTAs), ODE fits two particles
-// per thread (their RK4 losses packed) in CTAs sized by their steps, both split
+// per thread (their RK4 losses packed) in CTAs sized by their steps and, where
+// `large` long fits of many particles run together, by that number, both split
 // over up to 16 CTAs
-LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread = 8);
+LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread = 8, int large = 0,
+                           int sm_count = 0);
 // group swarms by (kind, T, C); order lists descriptor indices group by
 // group, longest estimated work first inside each group
 void batch_plan(const std::vector<BatchSwarm>& descs, int threads, int ppt, std::vector<int>* order,
-                std::vector<LaunchGroup>* groups, int spread = 8);
+                std::vector<LaunchGroup>* groups, int spread, int sm_count);
 // a batch of ODE fits alone, its units of work placed on the SMs by cost
 // (pps_ode_teams.cu): every fit's whole run in one cooperative launch.  *taken
 // false: nothing was launched (one CTA or cluster per fit is faster for these,

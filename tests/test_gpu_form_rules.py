@@ -1,6 +1,11 @@
 """Which form a call takes: short runs, batches of few iterations and mixed
 batches are no slower than in another form of the same work that the library
 has, and equal it bit for bit."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -8,6 +13,7 @@ from test_gpu_sync_parity import assert_state_equal
 
 pytestmark = pytest.mark.gpu
 
+PACKAGE = Path(__file__).resolve().parent.parent / "parallelparticleswarms.jl_gb300"
 GENERAL = dict(c1=1e-35, c2=1e-35)  # coefficients that only the general arithmetic takes
 
 
@@ -68,3 +74,51 @@ def test_batch_sampling(pps, count, n):
         assert np.array_equal(state[f], ref[f])
     if count <= 4:
         assert ms <= 1.3 * fixed + 0.02
+
+
+def _fit(pps, steps, seed=0):
+    data = np.linspace(0.5, 1.5, 2 * (steps // 10 + 1), dtype=np.float32).reshape(-1, 2) * (1.0 + 0.01 * seed)
+    return pps.ode.lv_problem(data.astype(np.float32), dt=0.01, nsteps=steps, save_every=10)
+
+
+@pytest.mark.parametrize("count", [1, 19, 20, 34, 35])
+@pytest.mark.parametrize("n", [4095, 4096, 8193])
+def test_large_fits_beside_a_swarm(pps, count, n):
+    with pps.Batch() as b:
+        for k in range(count):
+            b.add(_fit(pps, 40, k % 3), n, maxiters=2, seed=k % 3)
+        b.add(_problem(pps, "sphere", 4), 100, maxiters=2, seed=1)
+        b.run()
+        for k in range(min(count, 3)):
+            with pps.Swarm(_fit(pps, 40, k), n, seed=k) as sw:
+                sw.init().sync_run(2)
+                u, cost, idx = sw.gbest()
+            for slot in range(k, count, 3):
+                got = b.result(slot)
+                assert np.array_equal(got[0], u) and got[1:] == (cost, idx)
+
+
+MIXED = """
+import numpy as np
+import parallelparticleswarms as pps
+data = np.linspace(0.5, 1.5, 2 * 101, dtype=np.float32).reshape(-1, 2)
+fit = pps.ode.lv_problem(data, dt=0.01, nsteps=1000, save_every=10)
+small = pps.OptimizationProblem(pps.REGISTRY["sphere"], np.zeros(4, np.float32), None,
+                                lb=np.full(4, -3, np.float32), ub=np.full(4, 4, np.float32))
+with pps.Batch() as b:
+    b.set_shape(256, 1)
+    for k in range(24):
+        b.add(fit, 8192, maxiters=10, seed=k)
+    b.add(small, 100, maxiters=10, seed=1)
+    b.run()
+    print(min(b.run() for _ in range(5)))
+"""
+
+
+def test_time_of_large_fits_beside_a_swarm():
+    def ms(**env):
+        r = subprocess.run([sys.executable, "-c", MIXED], env=dict(os.environ, PYTHONPATH=str(PACKAGE), **env),
+                           capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr
+        return float(r.stdout)
+    assert ms() <= 1.1 * ms(PPS_ODE_THREADS="512")
