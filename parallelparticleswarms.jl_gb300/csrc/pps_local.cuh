@@ -174,7 +174,9 @@ __device__ __forceinline__ void lbfgs_run(const float* __restrict__ X0, int64_t 
       }
       stop = !ok;
       if (ok) {
-        if constexpr (OBJ == kUserObjective)
+        // (2-D Rosenbrock is faster with the whole evaluation: 20,000 particles, 50
+        // iterations, 133 us a call for 144)
+        if constexpr (OBJ == kUserObjective || (OBJ == kRosenbrock && MAXD == 2))
           fn = obj_grad<OBJ, MAXD>(op, xn, gn, D);
         else
           obj_gradient<OBJ, MAXD>(op, xn, gn, D, s1, s2);  // from the accepted point's value
