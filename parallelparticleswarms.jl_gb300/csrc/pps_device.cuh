@@ -279,8 +279,8 @@ __device__ __forceinline__ float cos2pi(float x) {
 // 1/4), and cos(2 pi x) is negative exactly where |f| > 1/4 (n odd above).
 // The polynomial is cos2pi's with z = 4 h^2 and its powers of two moved into
 // the constants and the last step, which changes no rounding: 4p = 1 - 16 h^2
-// is one fused multiply-add, c = 4p (z q / 4) + 4p.  Beyond 2^126 cos2pi's 2x
-// overflows and it returns NaN; this form would not.
+// is one fused multiply-add, c = 4p (z q / 4) + 4p.  From 2^127 on cos2pi's 2x
+// overflows and it returns NaN, which this form would not: the limit stays below.
 constexpr float kCosBoxLimit = 0x1p+126f;
 __device__ __forceinline__ float cos2pi_box(float x) {
   const float f = fabsf(__fsub_rn(x, rintf(x)));
