@@ -674,10 +674,15 @@ static bool brief_fit(const BatchSwarm& d) {
 // the SMs are full and small CTAs balance best.  Ms, ten iterations beside four
 // small swarms, 128 x 8 / 256 x 8 / 512 x 4: 8 LV fits of 8192 particles and 1000
 // steps 2.7 / 1.9 / 3.8, 16 of 16384 8.3 / 7.1 / 7.5, 24 of 8192 5.0 / 5.0 / 3.6, 24 FHN 6.2 /
-// 6.9 / 4.9, 38 FHN and 400 steps 3.5 / 3.6 / 4.0.
-constexpr int64_t kLargeFit = 4096;
-static bool large_fit(const BatchSwarm& d) { return is_ode(d.objective) && d.n >= kLargeFit && !brief_fit(d); }
-// `large`: how many such fits run together (0: not known)
+// 6.9 / 4.9, 38 FHN and 400 steps 3.5 / 3.6 / 4.0; us, one LV fit of 3000 and 600 steps with
+// a save each, six iterations 1170 / 725 / 1005.
+constexpr int64_t kLargeFit = 2048;  // more than one trip of eight CTAs of 128 threads
+static bool large_fit(const BatchSwarm& d) { return is_ode(d.objective) && d.n > kLargeFit && !brief_fit(d); }
+static int large_fits(const std::vector<BatchSwarm>& descs) {
+  int count = 0;
+  for (const auto& d : descs) count += large_fit(d);
+  return count;
+}
 static void ode_shape(const BatchSwarm& d, int large, int sm_count, int* threads, int* cluster) {
   const int given = ode_threads();
   bool wide = brief_fit(d) || given;
@@ -733,8 +738,7 @@ static int64_t chunk_of(int64_t n, int C, int width) { return cta_chunk(n, C, wi
 void batch_plan(const std::vector<BatchSwarm>& descs, int threads, int ppt, std::vector<int>* order,
                 std::vector<LaunchGroup>* groups, int spread, int sm_count) {
   const int ns = (int)descs.size();
-  int large = 0;
-  for (const auto& d : descs) large += large_fit(d);
+  const int large = large_fits(descs);
   std::map<std::tuple<int, int, int>, std::vector<int>> by;
   for (int k = 0; k < ns; ++k) {
     const LaunchGroup g = batch_group_of(descs[k], threads, ppt, spread, large, sm_count);
@@ -1165,7 +1169,9 @@ int pps_batch_run(pps_batch* b, float* device_ms) {
   b->last_ppt = ppt;
   if (all_ode) {
     b->last_threads = 0;
-    for (const auto& d : b->descs) b->last_threads = std::max(b->last_threads, batch_group_of(d, threads, ppt).T);
+    const int large = large_fits(b->descs);
+    for (const auto& d : b->descs)
+      b->last_threads = std::max(b->last_threads, batch_group_of(d, threads, ppt, spread, large, b->sm_count).T);
     b->last_ppt = 2;
   }
   b->last_spread = spread;

@@ -57,9 +57,9 @@ size_t batch_smem_bytes(int maxdim, int data_floats, int64_t maxchunk);
 // the (kind, T, C) a swarm is launched with: separable swarms use the
 // batch's block size and about `spread` particles per thread per iteration
 // (8 by default; fewer split a swarm over more CTAs), ODE fits two particles
-// per thread (their RK4 losses packed) in CTAs sized by their steps and, where
-// `large` long fits of many particles run together, by that number, both split
-// over up to 16 CTAs
+// per thread (their RK4 losses packed) in CTAs sized by their steps and by the
+// number `large` of long fits of many particles that run together (0: not known),
+// both split over up to 16 CTAs
 LaunchGroup batch_group_of(const BatchSwarm& d, int threads, int ppt, int spread = 8, int large = 0,
                            int sm_count = 0);
 // group swarms by (kind, T, C); order lists descriptor indices group by

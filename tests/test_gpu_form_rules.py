@@ -98,26 +98,44 @@ def test_large_fits_beside_a_swarm(pps, count, n):
                 assert np.array_equal(got[0], u) and got[1:] == (cost, idx)
 
 
+@pytest.mark.parametrize("every", [1, 2, 3, 4, 5, 6, 7, 10, 15, 60])
+@pytest.mark.parametrize("n", [300, 3000])
+def test_steps_between_saves(pps, every, n):
+    data = np.linspace(0.5, 1.5, 2 * (60 // every + 1), dtype=np.float32).reshape(-1, 2)
+    fit = pps.ode.fhn_problem(data, dt=0.02, nsteps=60, save_every=every)
+    with pps.Swarm(fit, n, seed=2) as sw, pps.Batch() as b:
+        sw.init().sync_run(3)
+        b.add(fit, n, maxiters=3, seed=2)
+        b.add(_problem(pps, "sphere", 4), 100, maxiters=3, seed=1)
+        b.run()
+        x, got = sw.state(), b.state(0)
+    for f in ("x", "pcost", "cost"):
+        assert np.array_equal(x[f], got[f]), f
+
+
 MIXED = """
+import sys
 import numpy as np
 import parallelparticleswarms as pps
-data = np.linspace(0.5, 1.5, 2 * 101, dtype=np.float32).reshape(-1, 2)
-fit = pps.ode.lv_problem(data, dt=0.01, nsteps=1000, save_every=10)
+count, n, steps, every = map(int, sys.argv[1:])
+data = np.linspace(0.5, 1.5, 2 * (steps // every + 1), dtype=np.float32).reshape(-1, 2)
+fit = pps.ode.lv_problem(data, dt=0.01, nsteps=steps, save_every=every)
 small = pps.OptimizationProblem(pps.REGISTRY["sphere"], np.zeros(4, np.float32), None,
                                 lb=np.full(4, -3, np.float32), ub=np.full(4, 4, np.float32))
 with pps.Batch() as b:
     b.set_shape(256, 1)
-    for k in range(24):
-        b.add(fit, 8192, maxiters=10, seed=k)
+    for k in range(count):
+        b.add(fit, n, maxiters=10, seed=k)
     b.add(small, 100, maxiters=10, seed=1)
     b.run()
     print(min(b.run() for _ in range(5)))
 """
 
 
-def test_time_of_large_fits_beside_a_swarm():
+@pytest.mark.parametrize("batch", [("24", "8192", "1000", "10"), ("1", "3000", "600", "1")])
+def test_time_of_large_fits_beside_a_swarm(batch):
     def ms(**env):
-        r = subprocess.run([sys.executable, "-c", MIXED], env=dict(os.environ, PYTHONPATH=str(PACKAGE), **env),
+        r = subprocess.run([sys.executable, "-c", MIXED, *batch], env=dict(os.environ, PYTHONPATH=str(PACKAGE), **env),
                            capture_output=True, text=True, timeout=300)
         assert r.returncode == 0, r.stderr
         return float(r.stdout)
