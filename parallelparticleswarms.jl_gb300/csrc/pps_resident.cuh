@@ -367,7 +367,9 @@ __device__ __forceinline__ void resident_run(const SwarmDev& s, const ObjParams&
     if (!none) src = (a.from_position || flag[lp]) ? X : P;
     // ---- agree on the global best
     const uint32_t seq = a.seq0 + 1u + (uint32_t)it;
-    const unsigned int limit = it == 0 ? a.start_limit : a.poll_limit;
+    // (a user objective's limits are the same, and the choice alone took its kernel
+    // from 1.97 to 2.32 ms for 200 iterations of 100,003 x 20-D)
+    const unsigned int limit = !ROWS && it == 0 ? a.start_limit : a.poll_limit;
     const int nb = a.blocks;
     unsigned long long* kw = a.xch + (size_t)par * resident_words(nb, D);  // keys
     unsigned long long* vw = kw + 2 * (size_t)nb;                          // vectors
