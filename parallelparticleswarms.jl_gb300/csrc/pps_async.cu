@@ -332,16 +332,16 @@ static int launch_async_obj(pps_swarm* s, int iters, float c1, float c2, int lan
   const PhiloxKeys keys = philox_round_keys(s->seed);
   const size_t smem = 3 * sizeof(float) * (size_t)lanes * slice;
   const float c1s = c1 * 0x1p-24f, c2s = c2 * 0x1p-24f;
-  // Blocks an SM (registers a thread): two, and three or four for slices of 4 to 8
-  // where the grid has more than one round of two and the run is short, or more
-  // than two rounds.  There the loads of the state count, which more warps
-  // overlap: 10^6 x 8-D sphere, us a run of 1 / 5 iterations, two blocks 115 / 156,
-  // three 90 / 122, k_async 91 / 132.  Few blocks gain nothing from the cap on registers:
-  // 10,000 x 8-D, 100 iterations, 72.5 with two, 80.8 with three.  Up to three
-  // iterations take k_async where that is so and where a slice has at most four dims: 10^6 x
-  // 5-D, one iteration 62, three blocks 67; 10,000 x 3-D 24 and 26.
+  // Blocks an SM (registers a thread): two, and in short runs three or four for
+  // slices of 4 to 8 where the grid has more than one round of two (two rounds for
+  // slices of 4).  There the loads of the state count, which more warps overlap: 10^6
+  // x 8-D sphere, us a run of 1 / 5 iterations, two blocks 115 / 156, three 90 / 122,
+  // k_async 91 / 132.  From ten to twenty iterations on the registers count for more:
+  // 300 iterations of 160,000 to 10^6 particles take 1 to 6 % longer with three or four.
+  // Up to three iterations take k_async where the grid is that long and where a slice has at
+  // most four dims: 10^6 x 5-D, one iteration 62, three blocks 67; 10,000 x 3-D 24 and 26.
   const int64_t round = 2 * (int64_t)s->sm_count;
-  const bool many = blocks > round && (iters <= 10 || blocks > 2 * round);
+  const bool many = iters <= 8 && blocks > (slice == 4 ? 2 : 1) * round;
 #define L_SLICE_B(S, B) \
   k_async_slice<OBJ, S, B><<<(unsigned)blocks, kAsyncThreads, smem, s->stream>>>(s->dv, s->op, keys, iters, c1s, c2s, lanes, 1.0f)
 #define L_SLICE(S)                                      \
